@@ -235,6 +235,10 @@ struct Context {
     int operator_levels = 0;
     bool operator_has32 = false;
     DArray<double> scratch;   // reductions
+    // grid-barrier counts and partial sums of the one-launch cycle (cycle.cu)
+    DArray<uint32_t> cycle_bar;
+    DArray<double> cycle_part;
+    int cycle_which = 0;
     double* host_scalars = nullptr;   // pinned
 
     bool profiling = false;

@@ -27,33 +27,11 @@
 #include <type_traits>
 
 #include "internal.cuh"
+#include "stencil.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace uwg {
-
-struct Grid {
-    int dim;
-    int64_t nx, ny, nz;  // nodes per axis
-    int64_t nn;
-    int ex, ey, ez;      // elements per axis
-};
-
-static Grid grid_of(const MeshDesc& m) {
-    Grid g;
-    g.dim = m.dim;
-    g.nx = m.nnx;
-    g.ny = m.nny;
-    g.nz = m.nnz;
-    g.nn = m.nn;
-    g.ex = m.nel[0];
-    g.ey = m.nel[1];
-    g.ez = m.dim == 3 ? m.nel[2] : 1;
-    return g;
-}
-
-template <int DIM>
-__host__ __device__ constexpr int nblocks() { return DIM == 3 ? 27 : 9; }
 
 // ------------------------------------------------------------------------------------------
 // Stencil build from packed element matrices (gather per node, 9 accumulators per block).
@@ -172,38 +150,6 @@ __global__ void k_convert(int64_t n, const S* __restrict__ a, D* __restrict__ b)
 // ------------------------------------------------------------------------------------------
 // Apply and smoothing.
 // ------------------------------------------------------------------------------------------
-// Neighbour offsets of node (i, j, k) per axis, 0 towards a missing neighbour.  Every stencil block
-// towards a neighbour outside the mesh is stored as zero, so a row reads the node itself there
-// and all loads of a row are unconditional (they can all be in flight at once).
-struct NbrOffsets {
-    int64_t dx[3], dy[3], dz[3];
-};
-
-template <int DIM>
-__device__ __forceinline__ NbrOffsets nbr_offsets(const Grid& g, int64_t i, int64_t j, int64_t k) {
-    NbrOffsets o;
-    o.dx[0] = i > 0 ? -1 : 0;
-    o.dx[1] = 0;
-    o.dx[2] = i + 1 < g.nx ? 1 : 0;
-    o.dy[0] = j > 0 ? -g.nx : 0;
-    o.dy[1] = 0;
-    o.dy[2] = j + 1 < g.ny ? g.nx : 0;
-    o.dz[0] = DIM == 3 && k > 0 ? -g.nx * g.ny : 0;
-    o.dz[1] = 0;
-    o.dz[2] = DIM == 3 && k + 1 < g.nz ? g.nx * g.ny : 0;
-    return o;
-}
-
-// (i, j, k) of node n with 32-bit division (node counts stay below 2^32, checked on the host)
-template <int DIM>
-__device__ __forceinline__ void node_ijk(const Grid& g, int64_t n, int64_t& i, int64_t& j, int64_t& k) {
-    const unsigned un = (unsigned)n, nx = (unsigned)g.nx, ny = (unsigned)g.ny;
-    const unsigned q = un / nx;
-    i = un - q * nx;
-    j = DIM == 3 ? q % ny : q;
-    k = DIM == 3 ? q / ny : 0;
-}
-
 // Row-split layout: a block of kRowThreads threads covers kRowThreads/DIM nodes; warp w works on
 // row w % DIM of 32 consecutive nodes (lanes), so every stencil load of a warp is coalesced and a
 // node's DIM rows run on DIM threads (three times the parallelism of one thread per node).
@@ -341,56 +287,23 @@ __global__ void __launch_bounds__(kRowThreads) k_apply(Grid g, const T* __restri
 
 // `sweeps` symmetric multicolour block Gauss-Seidel sweeps (colours ascending, then
 // descending) in one cooperative launch: x_n += Dinv_n (b_n - (A x)_n).  Nodes of one parity
-// colour are never stencil neighbours, so a colour is relaxed in parallel; the DIM row
-// residuals of a node meet in shared memory before its update, and a grid-wide barrier
-// separates colours.
+// colour are never stencil neighbours, so a colour is relaxed in parallel; a grid-wide barrier
+// separates colours.  The levels of the one-launch cycle (cycle.cu) do not come here.
 template <int DIM, typename T>
-__global__ void __launch_bounds__(kRowThreads) k_gs_sweeps(Grid g, const T* __restrict__ A, const T* __restrict__ Dinv,
-                                                           const T* __restrict__ b, T* __restrict__ x, int sweeps,
-                                                           int zero_init) {
-    __shared__ T sres[kRowThreads];
+__global__ void __launch_bounds__(kSplitThreads) k_gs_sweeps(Grid g, const T* __restrict__ A, const T* __restrict__ Dinv,
+                                                             const T* b, T* x, int sweeps, int zero_init) {
+    __shared__ T sres[2 * kSplitThreads];
     cg::grid_group grid = cg::this_grid();
-    constexpr int NPB = kRowThreads / DIM;
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int r = warp % DIM, grp = warp / DIM;
     if (zero_init) {
         const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
         const int64_t stride = (int64_t)gridDim.x * blockDim.x;
         for (int64_t t = tid; t < g.nn * DIM; t += stride) x[t] = (T)0;
         grid.sync();
     }
-    constexpr int NCOL = 1 << DIM;
-    for (int s = 0; s < sweeps; ++s) {
-        for (int step = 0; step < 2 * NCOL; ++step) {
-            int col = step < NCOL ? step : 2 * NCOL - 1 - step;
-            int px = col & 1, py = (col >> 1) & 1, pz = (col >> 2) & 1;
-            int64_t cx = (g.nx - px + 1) / 2, cy = (g.ny - py + 1) / 2;
-            int64_t cz = DIM == 3 ? (g.nz - pz + 1) / 2 : 1;
-            int64_t cnt = cx * cy * cz;
-            for (int64_t base = (int64_t)blockIdx.x * NPB; base < cnt; base += (int64_t)gridDim.x * NPB) {
-                int64_t t = base + grp * 32 + lane;
-                bool act = t < cnt;
-                int64_t n = 0;
-                T res = (T)0;
-                if (act) {
-                    int64_t i = 2 * (t % cx) + px, j = 2 * ((t / cx) % cy) + py;
-                    int64_t k = DIM == 3 ? 2 * (t / (cx * cy)) + pz : 0;
-                    n = i + g.nx * (j + g.ny * k);
-                    res = b[(int64_t)r * g.nn + n] - stencil_row_r<DIM, T>(g, n, i, j, k, r, A, x);
-                }
-                sres[threadIdx.x] = res;
-                __syncthreads();
-                if (act) {
-                    T v = x[(int64_t)r * g.nn + n];
-#pragma unroll
-                    for (int cc = 0; cc < DIM; ++cc)
-                        v = fma(Dinv[(int64_t)(r * DIM + cc) * g.nn + n], sres[(grp * DIM + cc) * 32 + lane], v);
-                    x[(int64_t)r * g.nn + n] = v;
-                }
-                __syncthreads();
-            }
-            grid.sync();
-        }
+    const int steps = gs_steps<DIM>(sweeps);
+    for (int step = 0; step < steps; ++step) {
+        if (step) grid.sync();
+        gs_colour<DIM, T>(g, A, Dinv, b, x, gs_step_colour<DIM>(step), blockIdx.x, gridDim.x, sres);
     }
 }
 
@@ -1036,12 +949,12 @@ void level_smooth(Context& c, const Level& L, const T* b, T* x, int sweeps, bool
         int per_sm = 0, sms = 0, dev = 0;
         UWG_CUDA(cudaGetDevice(&dev));
         UWG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        UWG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kRowThreads, 0));
+        UWG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSplitThreads, 0));
         UWG_REQUIRE(per_sm > 0, UWGPU_ERR_CUDA, "smoother kernel cannot be made resident");
         max_blocks[di][ti] = per_sm * sms;
     }
     int64_t per_colour = (g.nn + (1 << D) - 1) >> D;
-    int64_t npb = kRowThreads / D;
+    int64_t npb = D == 3 ? Split<3>::kNodes : Split<2>::kNodes;
     int64_t want = (per_colour + npb - 1) / npb;
     int blocks = (int)(want < max_blocks[di][ti] ? want : max_blocks[di][ti]);
     if (blocks < 1) blocks = 1;
@@ -1050,7 +963,7 @@ void level_smooth(Context& c, const Level& L, const T* b, T* x, int sweeps, bool
     int zi = zero_init ? 1 : 0;
     void* args[] = {(void*)&g, (void*)&A, (void*)&Di, (void*)&b, (void*)&x, (void*)&sweeps, (void*)&zi};
     LaunchScope ls(c, UWGPU_KERNEL_SMOOTH);
-    UWG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kRowThreads), args, 0, c.stream));
+    UWG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kSplitThreads), args, 0, c.stream));
 }
 
 template <typename T>

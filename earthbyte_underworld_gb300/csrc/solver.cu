@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "cycle.cuh"
 #include "internal.cuh"
 #include "unet.cuh"
 
@@ -332,6 +333,14 @@ struct Fgmres {
     template <typename Aop, typename Mop>
     int solve(Aop&& A, Mop&& M, const T* b, T* x, double rtol, int maxit, double* res_out, double* bnorm_out,
               bool* nan_out) {
+        return solve(A, M, [](int) { return false; }, b, x, rtol, maxit, res_out, bnorm_out, nan_out);
+    }
+
+    // fused(k): does the whole of iteration k (Z_k = M V_k, w = A Z_k, its orthogonalisation, V_{k+1}) and
+    // leaves H's column in host_scalars as cycle_fgmres_iteration describes, or returns false.
+    template <typename Aop, typename Mop, typename Fop>
+    int solve(Aop&& A, Mop&& M, Fop&& fused, const T* b, T* x, double rtol, int maxit, double* res_out,
+              double* bnorm_out, bool* nan_out) {
         hist.clear();
         zero<T>(c, n, x);
         double bnorm = red.norm<T>(n, b);
@@ -371,24 +380,33 @@ struct Fgmres {
                 T* vk = V.p + (int64_t)k * n;
                 T* zk = Z.p + (int64_t)k * n;
                 cycle_k = k;
-                M(vk, zk);
-                A(zk, w.p);
-                // CGS2
-                for (int pass = 0; pass < 2; ++pass) {
-                    red.multidot<T>(n, V.p, n, k + 1, w.p, hcol.data() + 0);
-                    UWG_CUDA(cudaMemcpyAsync(dvec.p, hcol.data(), (k + 1) * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-                    {
-                        LaunchScope ls(c, UWGPU_KERNEL_VECTOR);
-                        k_multi_axpy<T><<<blocks_for(n, 256), 256, 0, c.stream>>>(n, V.p, n, k + 1, dvec.p, w.p, -1.0);
+                double hn = 0.0;
+                if (fused(k)) {
+                    UWG_CUDA(cudaStreamSynchronize(c.stream));
+                    const double* hs = c.host_scalars;
+                    for (int j = 0; j <= k; ++j) H[(size_t)j * m + k] = hs[j] + hs[kCyPass + j];
+                    hn = std::sqrt(hs[2 * kCyPass] > 0 ? hs[2 * kCyPass] : 0.0);
+                    H[(size_t)(k + 1) * m + k] = hn;
+                } else {
+                    M(vk, zk);
+                    A(zk, w.p);
+                    // CGS2
+                    for (int pass = 0; pass < 2; ++pass) {
+                        red.multidot<T>(n, V.p, n, k + 1, w.p, hcol.data() + 0);
+                        UWG_CUDA(cudaMemcpyAsync(dvec.p, hcol.data(), (k + 1) * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+                        {
+                            LaunchScope ls(c, UWGPU_KERNEL_VECTOR);
+                            k_multi_axpy<T><<<blocks_for(n, 256), 256, 0, c.stream>>>(n, V.p, n, k + 1, dvec.p, w.p, -1.0);
+                        }
+                        for (int j = 0; j <= k; ++j) {
+                            if (pass == 0) H[(size_t)j * m + k] = hcol[j];
+                            else H[(size_t)j * m + k] += hcol[j];
+                        }
                     }
-                    for (int j = 0; j <= k; ++j) {
-                        if (pass == 0) H[(size_t)j * m + k] = hcol[j];
-                        else H[(size_t)j * m + k] += hcol[j];
-                    }
+                    hn = red.norm<T>(n, w.p);
+                    H[(size_t)(k + 1) * m + k] = hn;
+                    if (hn > 0.0) scale<T>(c, n, 1.0 / hn, w.p, V.p + (int64_t)(k + 1) * n);
                 }
-                double hn = red.norm<T>(n, w.p);
-                H[(size_t)(k + 1) * m + k] = hn;
-                if (hn > 0.0) scale<T>(c, n, 1.0 / hn, w.p, V.p + (int64_t)(k + 1) * n);
                 for (int j = 0; j < k; ++j) {
                     double t = cs[j] * H[(size_t)j * m + k] + sn[j] * H[(size_t)(j + 1) * m + k];
                     H[(size_t)(j + 1) * m + k] = -sn[j] * H[(size_t)j * m + k] + cs[j] * H[(size_t)(j + 1) * m + k];
@@ -484,6 +502,21 @@ struct Bsscr {
         nlev = c.nlevels;
         nv = c.mesh.nn * dim;
         if (o.smoother == UWGPU_SMOOTHER_CHEBYSHEV) estimate_lmax();
+        cyc = CycleOpts{o.smoother == UWGPU_SMOOTHER_CHEBYSHEV, o.smooth_down, o.smooth_up, o.mg_cycle};
+        cyc_first = cycle_first_level(c, cyc);
+    }
+    // the levels that one launch runs (cycle.cu)
+    CycleOpts cyc{};
+    int cyc_first = kMaxLevels;
+
+    // one FGMRES iteration of a velocity solve whose whole hierarchy is small
+    template <typename T>
+    bool fused_iteration(Fgmres<T>& gm, int k) {
+        if (cyc_first != 0 || learned_on) return false;
+        cycle_fgmres_iteration<T>(c, cyc, gm.V.p, k, nv, gm.Z.p + (int64_t)k * nv, gm.w.p,
+                                  gm.V.p + (int64_t)(k + 1) * nv, c.host_scalars);
+        rep.vcycles++;
+        return true;
     }
 
     // ---- learned correction of the V-cycle (unet.cu): M(r) = S(V(r) + N(r, V(r))) ----
@@ -566,6 +599,10 @@ struct Bsscr {
 
     template <typename T>
     void vcycle(int l, const T* b, T* x) {
+        if (l == cyc_first) {
+            cycle_run<T>(c, cyc, l, b, x);
+            return;
+        }
         Level& L = c.levels[l];
         if (l == nlev - 1) {
             if (nlev > 1)
@@ -605,7 +642,7 @@ struct Bsscr {
             learned_on = learned;
             its = gm64.solve([&](const double* in, double* out) { level_apply<double>(c, L0, in, out); },
                              [&](const double* in, double* out) { precondition<double>(in, out, gm64.hist, gm64.cycle_k); },
-                             b, x, rtol, maxit, &res, &bn, &nn);
+                             [&](int k) { return fused_iteration<double>(gm64, k); }, b, x, rtol, maxit, &res, &bn, &nn);
             if (nn) nan = true;
             if (!(res <= rtol * bn * 1.0000001) && bn > 0) inner_fail = true;
         } else {
@@ -626,7 +663,8 @@ struct Bsscr {
                 double inner_rtol = std::max(rtol * bn / rn, 1e-4);
                 int k = gm32.solve([&](const float* in, float* out) { level_apply<float>(c, L0, in, out); },
                                    [&](const float* in, float* out) { precondition<float>(in, out, gm32.hist, gm32.cycle_k); },
-                                   r32.p, d32.p, std::min(inner_rtol, 0.5), maxit - its, &res, &b32n, &nn);
+                                   [&](int k) { return fused_iteration<float>(gm32, k); }, r32.p, d32.p,
+                                   std::min(inner_rtol, 0.5), maxit - its, &res, &b32n, &nn);
                 its += k;
                 if (nn) { nan = true; break; }
                 {
@@ -1060,6 +1098,7 @@ void Bsscr::run() {
     if (c.has_bc && c.bc_nonzero) axpy<double>(c, nv, 1.0, ub.p, c.u_sol.p);
     UWG_CUDA(cudaStreamSynchronize(c.stream));
     if (learned) unet::check_errors(c, *c.net);
+    cycle_check(c);
     auto t2c = std::chrono::steady_clock::now();
     rep.t_solve_ms = std::chrono::duration<double, std::milli>(t2c - t1).count();
     c.has_solution = true;
@@ -1148,6 +1187,7 @@ int learned_generate(Context& c, const uwgpu_solve_opts& o, int nsamples, uint64
             if (s.red.norm<double>(nv, e.p) <= 1e-8 * un) break;
         }
     }
+    cycle_check(c);
     unet::dataset_finish(c, n);
     return n.nsamples;
 }

@@ -205,10 +205,8 @@ int uwgpu_solution_set(uwgpu_ctx* ctx, const double* u_nodal, const double* p) {
         UWG_REQUIRE(u_nodal && p, UWGPU_ERR_ARGUMENT, "null solution");
         int dim = c.mesh.dim;
         int64_t nn = c.mesh.nn;
-        std::vector<double> soa((size_t)nn * dim);
-        for (int64_t n = 0; n < nn; ++n)
-            for (int d = 0; d < dim; ++d) soa[(size_t)d * nn + n] = u_nodal[n * dim + d];
-        upload(c.u_sol, soa.data(), soa.size(), c.stream);
+        c.u_sol.ensure((size_t)nn * dim);
+        uwg::vector_from_host<double>(c, nn, dim, u_nodal, c.u_sol.p);
         upload(c.p_sol, p, (size_t)c.mesh.ne, c.stream);
         UWG_CUDA(cudaStreamSynchronize(c.stream));
         c.has_solution = true;
@@ -331,12 +329,7 @@ int uwgpu_bin_and_map(uwgpu_ctx* ctx, uint32_t* perm, uint32_t* offsets, double*
         if (perm && N) UWG_CUDA(cudaMemcpyAsync(perm, c.perm.p, N * sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
         if (offsets) UWG_CUDA(cudaMemcpyAsync(offsets, c.offsets.p, (E + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
         if (xi && N) {
-            std::vector<double> tmp(3 * N);
-            int dim = c.mesh.dim;
-            UWG_CUDA(cudaMemcpyAsync(tmp.data(), c.sxi.p, (size_t)dim * N * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-            UWG_CUDA(cudaStreamSynchronize(c.stream));
-            for (size_t s = 0; s < N; ++s)
-                for (int d = 0; d < 3; ++d) xi[3 * s + d] = d < dim ? tmp[(size_t)d * N + s] : 0.0;
+            uwg::vector_to_host<double>(c, c.np, c.mesh.dim, 3, c.sxi.p, xi);
         }
         UWG_CUDA(cudaStreamSynchronize(c.stream));
     });
@@ -360,38 +353,15 @@ int uwgpu_get_element_matrices(uwgpu_ctx* ctx, int64_t first, int64_t count, dou
         UWG_REQUIRE(c.assembled, UWGPU_ERR_STATE, "nothing assembled");
         int64_t E = c.mesh.ne;
         UWG_REQUIRE(first >= 0 && count >= 0 && first + count <= E, UWGPU_ERR_ARGUMENT, "element range");
-        int dim = c.mesh.dim, nen = dim == 3 ? 8 : 4, nd = nen * dim, np = uwg::packed_size(nd);
+        const int dim = c.mesh.dim, nd = dim << dim;
         if (count == 0) return;
-        auto fetch = [&](const double* base, int entries, std::vector<double>& out) {
-            out.resize((size_t)entries * count);
-            // entry-major [k][e]: one strided copy
-            UWG_CUDA(cudaMemcpy2DAsync(out.data(), count * sizeof(double), base + first, E * sizeof(double),
-                                       count * sizeof(double), entries, cudaMemcpyDeviceToHost, c.stream));
-        };
-        std::vector<double> hk, hf, hg;
         const bool full = c.assembled_jacobian;   // the Newton form's non-symmetric K_e, all entries
-        if (Ke) fetch(full ? c.Kjac.p : c.levels[0].Ke.p, full ? nd * nd : np, hk);
-        if (fe) fetch(c.fe.p, nd, hf);
-        if (Ge) fetch(c.Ge.p, nd, hg);
+        if (Ke && full) uwg::entries_to_host(c, nd * nd, E, first, count, c.Kjac.p, Ke);
+        else if (Ke) uwg::element_matrices_to_host(c, first, count, c.levels[0].Ke.p, Ke);
+        if (fe) uwg::entries_to_host(c, nd, E, first, count, c.fe.p, fe);
+        if (Ge) uwg::entries_to_host(c, nd, E, first, count, c.Ge.p, Ge);
         if (Se) UWG_CUDA(cudaMemcpyAsync(Se, c.Se.p + first, count * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
         UWG_CUDA(cudaStreamSynchronize(c.stream));
-        for (int64_t e = 0; e < count; ++e) {
-            if (Ke && full) {
-                for (int k = 0; k < nd * nd; ++k) Ke[e * nd * nd + k] = hk[(size_t)k * count + e];
-            } else if (Ke) {
-                double* K = Ke + e * nd * nd;
-                for (int r = 0; r < nd; ++r)
-                    for (int q = r; q < nd; ++q) {
-                        double v = hk[(size_t)uwg::packed_index(nd, r, q) * count + e];
-                        K[r * nd + q] = v;
-                        K[q * nd + r] = v;
-                    }
-            }
-            for (int k = 0; k < nd; ++k) {
-                if (fe) fe[e * nd + k] = hf[(size_t)k * count + e];
-                if (Ge) Ge[e * nd + k] = hg[(size_t)k * count + e];
-            }
-        }
     });
 }
 
@@ -413,18 +383,21 @@ int uwgpu_operator_apply(uwgpu_ctx* ctx, int32_t precision, const double* x, dou
         int64_t nn = c.mesh.nn;
         if (!c.operator_built || (precision == UWGPU_PREC_MIXED && !c.operator_has32))
             uwg::build_operator(c, c.operator_built ? c.operator_levels : 1, precision == UWGPU_PREC_MIXED);
-        std::vector<double> soa((size_t)nn * dim);
-        for (int64_t n = 0; n < nn; ++n)
-            for (int d = 0; d < dim; ++d) soa[(size_t)d * nn + n] = x[n * dim + d];
-        uwg::DArray<double> dx, dy;
-        dx.ensure(soa.size());
-        dy.ensure(soa.size());
-        UWG_CUDA(cudaMemcpyAsync(dx.p, soa.data(), soa.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-        uwg::apply_fine(c, precision == UWGPU_PREC_MIXED, dx.p, dy.p);
-        UWG_CUDA(cudaMemcpyAsync(soa.data(), dy.p, soa.size() * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+        uwg::Level& L = c.levels[0];
+        if (precision == UWGPU_PREC_MIXED) {
+            uwg::vector_from_host<float>(c, nn, dim, x, L.x32.p);
+            uwg::level_apply<float>(c, L, L.x32.p, L.r32.p);
+            uwg::vector_to_host<float>(c, nn, dim, dim, L.r32.p, y);
+        } else {
+            const size_t nv = (size_t)nn * dim;
+            c.io_x.ensure(nv);
+            c.io_y.ensure(nv);
+            uwg::vector_from_host<double>(c, nn, dim, x, c.io_x.p);
+            uwg::level_apply<double>(c, L, c.io_x.p, c.io_y.p);
+            uwg::vector_to_host<double>(c, nn, dim, dim, c.io_y.p, y);
+        }
+        uwg::check_launch("operator apply");
         UWG_CUDA(cudaStreamSynchronize(c.stream));
-        for (int64_t n = 0; n < nn; ++n)
-            for (int d = 0; d < dim; ++d) y[n * dim + d] = soa[(size_t)d * nn + n];
     });
 }
 
@@ -463,13 +436,7 @@ int uwgpu_solve_bsscr(uwgpu_ctx* ctx, const uwgpu_solve_opts* opts, double* u, d
         uwg::solve_bsscr(c, o, rep);
         int dim = c.mesh.dim;
         int64_t nn = c.mesh.nn;
-        if (u) {
-            std::vector<double> soa((size_t)nn * dim);
-            UWG_CUDA(cudaMemcpyAsync(soa.data(), c.u_sol.p, soa.size() * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-            UWG_CUDA(cudaStreamSynchronize(c.stream));
-            for (int64_t n = 0; n < nn; ++n)
-                for (int d = 0; d < dim; ++d) u[n * dim + d] = soa[(size_t)d * nn + n];
-        }
+        if (u) uwg::vector_to_host<double>(c, nn, dim, dim, c.u_sol.p, u);
         if (p) UWG_CUDA(cudaMemcpyAsync(p, c.p_sol.p, c.mesh.ne * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
         UWG_CUDA(cudaStreamSynchronize(c.stream));
         if (report) *report = rep;
@@ -490,13 +457,7 @@ int uwgpu_solve_picard(uwgpu_ctx* ctx, const uwgpu_solve_opts* opts, double tole
         uwg::solve_picard(c, o, tolerance, max_iterations, min_iterations, rep, its, res);
         int dim = c.mesh.dim;
         int64_t nn = c.mesh.nn;
-        if (u) {
-            std::vector<double> soa((size_t)nn * dim);
-            UWG_CUDA(cudaMemcpyAsync(soa.data(), c.u_sol.p, soa.size() * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-            UWG_CUDA(cudaStreamSynchronize(c.stream));
-            for (int64_t n = 0; n < nn; ++n)
-                for (int d = 0; d < dim; ++d) u[n * dim + d] = soa[(size_t)d * nn + n];
-        }
+        if (u) uwg::vector_to_host<double>(c, nn, dim, dim, c.u_sol.p, u);
         if (p) UWG_CUDA(cudaMemcpyAsync(p, c.p_sol.p, c.mesh.ne * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
         UWG_CUDA(cudaStreamSynchronize(c.stream));
         if (report) *report = rep;

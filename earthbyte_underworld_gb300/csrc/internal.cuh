@@ -239,6 +239,8 @@ struct Context {
     DArray<uint32_t> cycle_bar;
     DArray<double> cycle_part;
     int cycle_which = 0;
+    DArray<double> io;        // staging of transfers to and from the host (hostio.cu)
+    DArray<double> io_x, io_y;   // vectors of uwgpu_operator_apply
     double* host_scalars = nullptr;   // pinned
 
     bool profiling = false;
@@ -368,12 +370,16 @@ inline unsigned blocks_for(int64_t n, int threads) {
 }
 
 // ---- functions shared between translation units ----
+// layout changes at the boundary to host memory (hostio.cu)
+template <typename T> void vector_from_host(Context& c, int64_t n, int dim, const double* host, T* soa);
+template <typename T> void vector_to_host(Context& c, int64_t n, int dim, int width, const T* soa, double* host);
+void entries_to_host(Context& c, int entries, int64_t ne, int64_t first, int64_t count, const double* src, double* host);
+void element_matrices_to_host(Context& c, int64_t first, int64_t count, const double* Kp, double* host);
 void bin_and_map(Context& c);
 void assemble(Context& c);
 void strain_weakening_advance(Context& c, double dt);
 int64_t population_control(Context& c, const uwgpu_pcdvc_opts& o);
 void build_operator(Context& c, int levels, bool need32);
-void apply_fine(Context& c, bool fp32, const double* x, double* y);  // device SoA vectors
 void solve_bsscr(Context& c, const uwgpu_solve_opts& o, uwgpu_report& rep);
 void estimate_fine_lmax(Context& c, const uwgpu_solve_opts& o);
 void weights_set(Context& c, int kind, const int32_t res[3]);

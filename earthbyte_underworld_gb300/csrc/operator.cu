@@ -1087,25 +1087,6 @@ template void level_prolong_add<float>(Context&, const Level&, const Level&, con
 template void level_coarse_solve<double>(Context&, const Level&, const double*, double*);
 template void level_coarse_solve<float>(Context&, const Level&, const float*, float*);
 
-void apply_fine(Context& c, bool fp32, const double* x, double* y) {
-    Level& L = c.levels[0];
-    if (!fp32) {
-        level_apply<double>(c, L, x, y);
-    } else {
-        size_t nv = (size_t)L.mesh.nn * L.mesh.dim;
-        {
-            LaunchScope ls(c, -1);
-            k_convert<double, float><<<blocks_for((int64_t)nv, 256), 256, 0, c.stream>>>((int64_t)nv, x, L.x32.p);
-        }
-        level_apply<float>(c, L, L.x32.p, L.r32.p);
-        {
-            LaunchScope ls(c, -1);
-            k_convert<float, double><<<blocks_for((int64_t)nv, 256), 256, 0, c.stream>>>((int64_t)nv, L.r32.p, y);
-        }
-    }
-    check_launch("apply_fine");
-}
-
 // ------------------------------------------------------------------------------------------
 // Gradient operators on the fine level (P0 pressure).
 // G_e[a][d] = -s_{d,a} * prod_{q != d} h_q / 2^(dim-1): the 2^dim-point Gauss integral of

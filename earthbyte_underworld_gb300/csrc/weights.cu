@@ -301,11 +301,8 @@ void integration_points_download(Context& c, double* xi, double* w) {
     if (N == 0) return;
     const double* src = c.weights_kind == UWGPU_WEIGHTS_DVC ? c.dvc_xi.p : c.sxi.p;
     if (xi) {
-        std::vector<double> tmp((size_t)dim * N);
-        UWG_CUDA(cudaMemcpyAsync(tmp.data(), src, tmp.size() * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+        vector_to_host<double>(c, (int64_t)N, dim, 3, src, xi);
         UWG_CUDA(cudaStreamSynchronize(c.stream));
-        for (size_t s = 0; s < N; ++s)
-            for (int d = 0; d < 3; ++d) xi[3 * s + d] = d < dim ? tmp[(size_t)d * N + s] : 0.0;
     }
     if (w) {
         if (c.weights_kind == UWGPU_WEIGHTS_DVC) {

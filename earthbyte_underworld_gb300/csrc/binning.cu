@@ -8,77 +8,84 @@
 //   local coords     StgFEM/Discretisation/src/ElementType.c:227-350 (Newton; on the affine
 //                    elements of a regular mesh it reproduces the closed form used here)
 //
-// GPU design: counting sort with integer atomics on HBM-resident counts, an exclusive scan,
+// GPU design: counting sort with integer atomics on HBM-resident counts (the count an atomic returns is
+// the point's place in its element, so the scatter needs no second atomic), an exclusive scan,
 // an unordered scatter, then one warp per element ranks its points by index so the final
 // permutation equals the reference's append order exactly.  The same warp computes xi and
 // gathers the per-point inputs into slot order (SoA), so assembly reads them coalesced.
+#include <cstring>
+
 #include "internal.cuh"
+#include "locate.cuh"
 
 namespace uwg {
 
 struct MeshParams {
-    int dim;
-    int nel[3];
-    double min[3];
-    double max[3];
+    AxisMap ax[3];
+    const double* tab[3];   // per axis: lower node x0[nel], width h[nel], 1/h[nel] of every element layer
 };
 
-static MeshParams params_of(const MeshDesc& m) {
-    MeshParams p;
-    p.dim = m.dim;
+// x0, h, RN(1/h) of the element layers of one axis
+__global__ void k_axis_table(int nel, double mn, double mx, double* __restrict__ tab) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nel) return;
+    const double x0 = node_coord_1d(i, nel, mn, mx), x1 = node_coord_1d(i + 1, nel, mn, mx);
+    const double h = x1 - x0;
+    tab[i] = x0;
+    tab[nel + i] = h;
+    tab[2 * nel + i] = __drcp_rn(h);
+}
+
+void axis_tables(Context& c, const double* tab[3]) {
+    const MeshDesc& m = c.mesh;
+    int64_t off[3], total = 0;
     for (int d = 0; d < 3; ++d) {
-        p.nel[d] = m.nel[d];
-        p.min[d] = m.min[d];
-        p.max[d] = m.max[d];
+        off[d] = d < m.dim ? total : 0;
+        if (d < m.dim) total += 3 * (int64_t)m.nel[d];
     }
+    if (!c.axis_tab_ok) {   // once per mesh
+        c.axis_tab.ensure((size_t)total);
+        for (int d = 0; d < m.dim; ++d) {
+            LaunchScope ls(c, UWGPU_KERNEL_BINNING);
+            k_axis_table<<<blocks_for(m.nel[d], 128), 128, 0, c.stream>>>(m.nel[d], m.min[d], m.max[d], c.axis_tab.p + off[d]);
+        }
+        check_launch("k_axis_table");
+        c.axis_tab_ok = true;
+    }
+    for (int d = 0; d < 3; ++d) tab[d] = c.axis_tab.p + off[d];
+}
+
+static MeshParams params_of(Context& c) {
+    MeshParams p;
+    for (int d = 0; d < 3; ++d) p.ax[d] = axis_map(c.mesh.min[d], c.mesh.max[d], c.mesh.nel[d]);
+    axis_tables(c, p.tab);
     return p;
 }
 
-__device__ __forceinline__ bool num_approx(double var, double val) {
-    const double eps = 1e-12;
-    return var >= val - eps && var <= val + eps;
-}
-
+// element of every point, its place in the element (in the order of the atomics) and the counts
 template <int DIM>
 __global__ void k_locate(int64_t np, const double* __restrict__ px, const double* __restrict__ py,
-                         const double* __restrict__ pz, MeshParams mp, uint32_t* __restrict__ cell,
-                         uint32_t* __restrict__ counts, uint32_t* __restrict__ err) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                         const double* __restrict__ pz, const __grid_constant__ MeshParams mp, uint32_t* __restrict__ cell,
+                         uint32_t* __restrict__ place, uint32_t* __restrict__ counts, uint32_t* __restrict__ err) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np) return;
-    double pt[3];
-    pt[0] = px[p];
-    pt[1] = py[p];
-    pt[2] = DIM == 3 ? pz[p] : 0.0;
-    unsigned inds[3] = {0u, 0u, 0u};
+    const double pt[3] = {px[p], py[p], DIM == 3 ? pz[p] : 0.0};
+    unsigned e = 0, mul = 1;
     bool ok = true;
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
-        double sep = (mp.max[d] - mp.min[d]) / mp.nel[d];
-        if (!isfinite(pt[d])) {
-            ok = false;
-        } else if (num_approx(pt[d] - mp.max[d], 0.0)) {
-            inds[d] = (unsigned)(mp.nel[d] - 1);
-        } else if (pt[d] < mp.min[d] || pt[d] > mp.max[d]) {
-            ok = false;
-        } else {
-            double out = __ddiv_rn(pt[d] - mp.min[d], sep);
-            double integer = trunc(out);
-            double frac = out - integer;  // exact: modf of a non-negative value
-            unsigned i = (unsigned)integer;
-            if (i > 0 && num_approx(frac, 0.0)) i--;
-            // a value that rounds onto the upper face is still inside the last element
-            if (i >= (unsigned)mp.nel[d]) i = (unsigned)mp.nel[d] - 1;
-            inds[d] = i;
-        }
+        int i = 0;
+        ok = axis_index(mp.ax[d], pt[d], i) && ok;
+        e += mul * (unsigned)i;
+        mul *= (unsigned)mp.ax[d].nel;
     }
     if (!ok) {
         cell[p] = 0xffffffffu;
         atomicAdd(err, 1u);
         return;
     }
-    unsigned e = inds[0] + (unsigned)mp.nel[0] * (inds[1] + (unsigned)mp.nel[1] * inds[2]);
     cell[p] = e;
-    atomicAdd(&counts[e], 1u);
+    place[p] = atomicAdd(&counts[e], 1u);
 }
 
 // ---- exclusive scan of u32 counts: out[0..n] with out[n] = total ----
@@ -154,7 +161,38 @@ __global__ void k_scan_add(int64_t n, uint32_t* __restrict__ out, const uint32_t
     if (i < n) out[i] += tile_sums[i / kScanTile];
 }
 
+// The whole scan in one block, for the element counts of small meshes (one launch of 2 us instead of three)
+constexpr int64_t kScanSmall = 2 * 1024 * kScanItems;
+
+__global__ void __launch_bounds__(1024) k_scan_small(int64_t n, const uint32_t* __restrict__ in, uint32_t* __restrict__ out) {
+    __shared__ uint32_t sw[32];
+    uint32_t carry = 0;
+    for (int64_t t = 0; t < n; t += 1024 * kScanItems) {
+        const int64_t base = t + (int64_t)threadIdx.x * kScanItems;
+        uint32_t v[kScanItems], s = 0, total;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            v[i] = (base + i < n) ? in[base + i] : 0u;
+            s += v[i];
+        }
+        uint32_t pre = carry + block_exclusive_scan(s, sw, total);
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            if (base + i < n) out[base + i] = pre;
+            pre += v[i];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) out[n] = carry;
+}
+
 static void exclusive_scan(Context& c, const uint32_t* in, uint32_t* out, int64_t n) {
+    if (n <= kScanSmall) {
+        LaunchScope ls(c, UWGPU_KERNEL_BINNING);
+        k_scan_small<<<1, 1024, 0, c.stream>>>(n, in, out);
+        check_launch("k_scan_small");
+        return;
+    }
     int64_t ntiles = (n + kScanTile - 1) / kScanTile;
     if (ntiles < 1) ntiles = 1;
     c.block_sums.ensure((size_t)ntiles);
@@ -175,74 +213,66 @@ static void exclusive_scan(Context& c, const uint32_t* in, uint32_t* out, int64_
     check_launch("k_scan_add");
 }
 
-__global__ void k_scatter(int64_t np, const uint32_t* __restrict__ cell, const uint32_t* __restrict__ offsets,
-                          uint32_t* __restrict__ cursor, uint32_t* __restrict__ tmp_perm) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_scatter(int64_t np, const uint32_t* __restrict__ cell, const uint32_t* __restrict__ place,
+                          const uint32_t* __restrict__ offsets, uint32_t* __restrict__ tmp_perm) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np) return;
-    uint32_t e = cell[p];
+    const uint32_t e = cell[p];
     if (e == 0xffffffffu) return;
-    uint32_t slot = offsets[e] + atomicAdd(&cursor[e], 1u);
-    tmp_perm[slot] = (uint32_t)p;
-}
-
-template <int DIM>
-__device__ __forceinline__ void map_point(int64_t e, uint32_t p, uint32_t slot, int64_t nslots, const MeshParams& mp,
-                                          const double* __restrict__ px, const double* __restrict__ py,
-                                          const double* __restrict__ pz, const int32_t* __restrict__ pmat,
-                                          const double* __restrict__ peta, const double* __restrict__ prho,
-                                          double* __restrict__ sxi, int32_t* __restrict__ smat,
-                                          double* __restrict__ seta, double* __restrict__ srho) {
-    int64_t ie = e % mp.nel[0];
-    int64_t je = (e / mp.nel[0]) % mp.nel[1];
-    int64_t ke = DIM == 3 ? e / ((int64_t)mp.nel[0] * mp.nel[1]) : 0;
-    int64_t idx[3] = {ie, je, ke};
-    double x[3] = {px[p], py[p], DIM == 3 ? pz[p] : 0.0};
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-        double x0 = node_coord_1d(idx[d], mp.nel[d], mp.min[d], mp.max[d]);
-        double x1 = node_coord_1d(idx[d] + 1, mp.nel[d], mp.min[d], mp.max[d]);
-        double h = x1 - x0;
-        sxi[(int64_t)d * nslots + slot] = (2.0 * (x[d] - x0) - h) / h;
-    }
-    smat[slot] = pmat[p];
-    if (seta) seta[slot] = peta[p];
-    if (srho) srho[slot] = prho[p];
+    tmp_perm[offsets[e] + place[p]] = (uint32_t)p;
 }
 
 // One warp per element: rank the element's points by point index (the append order of the
 // reference cell table), write the permutation, then map every point of the element.
+// xi = RN((2 (x - x0) - h) / h): the division by h is a product with RN(1/h) and one FMA correction, which
+// gives the correctly rounded quotient (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34, 1990): 5 FP64 instructions per axis where two divisions for
+// the node coordinates and one for xi took over 30, which bound this kernel (2.4M points: 556 us before).
 template <int DIM>
-__global__ void k_sort_map(int64_t ne, int64_t nslots, MeshParams mp, const uint32_t* __restrict__ offsets,
-                           const uint32_t* __restrict__ tmp_perm, uint32_t* __restrict__ perm,
-                           const double* __restrict__ px, const double* __restrict__ py,
-                           const double* __restrict__ pz, const int32_t* __restrict__ pmat,
-                           const double* __restrict__ peta, const double* __restrict__ prho,
-                           double* __restrict__ sxi, int32_t* __restrict__ smat, double* __restrict__ seta,
-                           double* __restrict__ srho) {
-    int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(256) k_sort_map(int64_t ne, int64_t nslots, const __grid_constant__ MeshParams mp,
+                                                  const uint32_t* __restrict__ offsets,
+                                                  const uint32_t* __restrict__ tmp_perm, uint32_t* __restrict__ perm,
+                                                  const double* __restrict__ px, const double* __restrict__ py,
+                                                  const double* __restrict__ pz, const int32_t* __restrict__ pmat,
+                                                  const double* __restrict__ peta, const double* __restrict__ prho,
+                                                  double* __restrict__ sxi, int32_t* __restrict__ smat,
+                                                  double* __restrict__ seta, double* __restrict__ srho) {
+    const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (e >= ne) return;
-    uint32_t beg = offsets[e], end = offsets[e + 1];
-    uint32_t n = end - beg;
-    if (n <= 32) {
-        uint32_t v = lane < (int)n ? tmp_perm[beg + lane] : 0xffffffffu;
-        int rank = 0;
+    const uint32_t beg = offsets[e], n = offsets[e + 1] - beg;
+    double x0[3], h[3], rh[3];
+    unsigned q = (unsigned)e;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            uint32_t o = __shfl_sync(0xffffffffu, v, j);
-            rank += (o < v) ? 1 : 0;
+    for (int d = 0; d < DIM; ++d) {
+        const int nel = mp.ax[d].nel;
+        const int i = d + 1 < DIM ? (int)(q % (unsigned)nel) : (int)q;
+        q /= (unsigned)nel;
+        x0[d] = __ldg(mp.tab[d] + i);
+        h[d] = __ldg(mp.tab[d] + nel + i);
+        rh[d] = __ldg(mp.tab[d] + 2 * nel + i);
+    }
+    for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+        const bool mine = i0 + lane < n;
+        const uint32_t v = mine ? tmp_perm[beg + i0 + lane] : 0xffffffffu;
+        uint32_t rank = 0;
+        for (uint32_t j0 = 0; j0 < n; j0 += 32) {
+            const uint32_t w = j0 == i0 ? v : (j0 + lane < n ? tmp_perm[beg + j0 + lane] : 0xffffffffu);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) rank += __shfl_sync(0xffffffffu, w, j) < v ? 1u : 0u;
         }
-        if (lane < (int)n) {
-            perm[beg + rank] = v;
-            map_point<DIM>(e, v, beg + rank, nslots, mp, px, py, pz, pmat, peta, prho, sxi, smat, seta, srho);
-        }
-    } else {
-        for (uint32_t i = lane; i < n; i += 32) {
-            uint32_t v = tmp_perm[beg + i];
-            uint32_t rank = 0;
-            for (uint32_t j = 0; j < n; ++j) rank += (tmp_perm[beg + j] < v) ? 1u : 0u;
-            perm[beg + rank] = v;
-            map_point<DIM>(e, v, beg + rank, nslots, mp, px, py, pz, pmat, peta, prho, sxi, smat, seta, srho);
+        if (!mine) continue;
+        const uint32_t slot = beg + rank;
+        const double x[3] = {px[v], py[v], DIM == 3 ? pz[v] : 0.0};
+        perm[slot] = v;
+        smat[slot] = pmat[v];
+        if (seta) seta[slot] = peta[v];
+        if (srho) srho[slot] = prho[v];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            const double a = fma(2.0, x[d] - x0[d], -h[d]);
+            const double t = a * rh[d];
+            sxi[(int64_t)d * nslots + slot] = fma(fma(-t, h[d], a), rh[d], t);
         }
     }
 }
@@ -251,44 +281,42 @@ void bin_and_map(Context& c) {
     UWG_REQUIRE(c.has_mesh, UWGPU_ERR_STATE, "mesh not set");
     UWG_REQUIRE(c.has_points, UWGPU_ERR_STATE, "material points not uploaded");
     const int64_t np = c.np, ne = c.mesh.ne;
-    MeshParams mp = params_of(c.mesh);
+    const MeshParams mp = params_of(c);
     c.cell.ensure((size_t)np);
-    c.counts.ensure((size_t)ne);
-    c.cursor.ensure((size_t)ne);
+    c.counts.ensure((size_t)ne + 1);   // and the number of points outside
+    c.place.ensure((size_t)np);
     c.offsets.ensure((size_t)ne + 1);
     c.perm.ensure((size_t)np);
     c.tmp_perm.ensure((size_t)np);
-    c.err_count.ensure(1);
     c.sxi.ensure((size_t)np * c.mesh.dim);
     c.smat.ensure((size_t)np);
     c.seta_out.ensure((size_t)np);
     if (c.has_peta) c.seta_in.ensure((size_t)np);
     if (c.has_prho) c.srho_in.ensure((size_t)np);
-    UWG_CUDA(cudaMemsetAsync(c.counts.p, 0, ne * sizeof(uint32_t), c.stream));
-    UWG_CUDA(cudaMemsetAsync(c.cursor.p, 0, ne * sizeof(uint32_t), c.stream));
-    UWG_CUDA(cudaMemsetAsync(c.err_count.p, 0, sizeof(uint32_t), c.stream));
+    uint32_t* err = c.counts.p + ne;
+    UWG_CUDA(cudaMemsetAsync(c.counts.p, 0, (ne + 1) * sizeof(uint32_t), c.stream));
     {
         // algorithmic bytes of the whole binning pass: per point coordinates read twice (locate,
-        // map), cell id written/read, count/cursor atomics, unordered and final permutation,
-        // material in, xi and material out (+ optional per-point inputs); per element counts,
-        // cursor and offsets
+        // map), cell id and place written/read, count atomics, unordered and final permutation,
+        // material in, xi and material out (+ optional per-point inputs); per element counts
+        // and offsets
         int dim = c.mesh.dim;
         double extra = (c.has_peta ? 16.0 : 0.0) + (c.has_prho ? 16.0 : 0.0);
-        double per_point = 2 * dim * 8.0 + 8.0 + 16.0 + 12.0 + 8.0 + dim * 8.0 + extra;
-        note_work(c, UWGPU_KERNEL_BINNING, per_point * np + 20.0 * ne, 0.0);
+        double per_point = 2 * dim * 8.0 + 16.0 + 16.0 + 12.0 + 8.0 + dim * 8.0 + extra;
+        note_work(c, UWGPU_KERNEL_BINNING, per_point * np + 16.0 * ne, 0.0);
     }
     if (np > 0) {
         LaunchScope ls(c, UWGPU_KERNEL_BINNING);
         if (c.mesh.dim == 3)
-            k_locate<3><<<blocks_for(np, 256), 256, 0, c.stream>>>(np, c.px.p, c.py.p, c.pz.p, mp, c.cell.p, c.counts.p, c.err_count.p);
+            k_locate<3><<<blocks_for(np, 256), 256, 0, c.stream>>>(np, c.px.p, c.py.p, c.pz.p, mp, c.cell.p, c.place.p, c.counts.p, err);
         else
-            k_locate<2><<<blocks_for(np, 256), 256, 0, c.stream>>>(np, c.px.p, c.py.p, nullptr, mp, c.cell.p, c.counts.p, c.err_count.p);
+            k_locate<2><<<blocks_for(np, 256), 256, 0, c.stream>>>(np, c.px.p, c.py.p, nullptr, mp, c.cell.p, c.place.p, c.counts.p, err);
     }
     check_launch("k_locate");
     exclusive_scan(c, c.counts.p, c.offsets.p, ne);
     if (np > 0) {
         LaunchScope ls(c, UWGPU_KERNEL_BINNING);
-        k_scatter<<<blocks_for(np, 256), 256, 0, c.stream>>>(np, c.cell.p, c.offsets.p, c.cursor.p, c.tmp_perm.p);
+        k_scatter<<<blocks_for(np, 256), 256, 0, c.stream>>>(np, c.cell.p, c.place.p, c.offsets.p, c.tmp_perm.p);
     }
     check_launch("k_scatter");
     {
@@ -304,9 +332,10 @@ void bin_and_map(Context& c) {
                                                        nullptr, c.pmat.p, c.peta.p, c.prho.p, c.sxi.p, c.smat.p, seta, srho);
     }
     check_launch("k_sort_map");
-    uint32_t outside = 0;
-    UWG_CUDA(cudaMemcpyAsync(&outside, c.err_count.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
+    UWG_CUDA(cudaMemcpyAsync(c.host_scalars, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
     UWG_CUDA(cudaStreamSynchronize(c.stream));
+    uint32_t outside = 0;
+    std::memcpy(&outside, c.host_scalars, sizeof(outside));
     c.mapped = true;
     c.assembled = false;
     if (outside)

@@ -128,6 +128,7 @@ int uwgpu_mesh_q1(uwgpu_ctx* ctx, int32_t dim, const int32_t nel[3], const doubl
         c.mesh = m;
         c.has_mesh = true;
         c.elem_h_for = -1;
+        c.axis_tab_ok = false;
         c.has_bc = false;
         c.mapped = false;
         c.assembled = false;

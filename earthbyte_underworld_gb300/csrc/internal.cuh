@@ -196,7 +196,9 @@ struct Context {
     bool has_points = false;
 
     // binning / mapping
-    DArray<uint32_t> cell, counts, offsets, cursor, perm, tmp_perm, block_sums;
+    DArray<uint32_t> cell, counts, offsets, place, perm, tmp_perm, block_sums;
+    DArray<double> axis_tab;   // node coordinates and widths of the element layers (binning.cu), once per mesh
+    bool axis_tab_ok = false;
     DArray<uint32_t> err_count;
     DArray<double> sxi;       // [d][slot]
     // integration weights: constant 2^dim / count, or discrete Voronoi cells of dvc_res cells
@@ -375,6 +377,7 @@ template <typename T> void vector_from_host(Context& c, int64_t n, int dim, cons
 template <typename T> void vector_to_host(Context& c, int64_t n, int dim, int width, const T* soa, double* host);
 void entries_to_host(Context& c, int entries, int64_t ne, int64_t first, int64_t count, const double* src, double* host);
 void element_matrices_to_host(Context& c, int64_t first, int64_t count, const double* Kp, double* host);
+void axis_tables(Context& c, const double* tab[3]);   // per axis x0[nel], h[nel], 1/h[nel] (binning.cu)
 void bin_and_map(Context& c);
 void assemble(Context& c);
 void strain_weakening_advance(Context& c, double dt);

@@ -23,6 +23,7 @@
 #include <mutex>
 
 #include "internal.cuh"
+#include "locate.cuh"
 
 namespace uwg_noalloc {
 
@@ -43,45 +44,28 @@ static uint32_t* g_addr[kMaxDevices];
 static std::mutex g_lock;
 
 struct MeshP {
+    uwg::AxisMap ax[3];
     int nel[3];
     double min[3], max[3];
 };
 
-__device__ __forceinline__ bool approx0(double v) { return v >= -1e-12 && v <= 1e-12; }
-
-// Element of each point (Mesh_RegularAlgorithms_SearchElements rule) and per-element counts.
+// Element of each point (Mesh_RegularAlgorithms_SearchElements rule, locate.cuh) and per-element counts.
 template <int DIM>
 __global__ void k_na_locate(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
                             const double* __restrict__ z, MeshP mp, uint32_t* __restrict__ s) {
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
-    double pt[3] = {x[p], y[p], DIM == 3 ? z[p] : 0.0};
-    unsigned ind[3] = {0u, 0u, 0u};
+    const double pt[3] = {x[p], y[p], DIM == 3 ? z[p] : 0.0};
+    int ind[3] = {0, 0, 0};
     bool ok = true;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-        double sep = (mp.max[d] - mp.min[d]) / mp.nel[d];
-        if (!isfinite(pt[d])) {
-            ok = false;
-        } else if (approx0(pt[d] - mp.max[d])) {
-            ind[d] = (unsigned)(mp.nel[d] - 1);
-        } else if (pt[d] < mp.min[d] || pt[d] > mp.max[d]) {
-            ok = false;
-        } else {
-            double out = (pt[d] - mp.min[d]) / sep;
-            double whole = trunc(out);
-            unsigned i = (unsigned)whole;
-            if (i > 0 && approx0(out - whole)) i--;
-            if (i >= (unsigned)mp.nel[d]) i = (unsigned)mp.nel[d] - 1;
-            ind[d] = i;
-        }
-    }
+    for (int d = 0; d < DIM; ++d) ok = uwg::axis_index(mp.ax[d], pt[d], ind[d]) && ok;
     if (!ok) {
         s[kOffCell + p] = 0xffffffffu;
         atomicAdd(&s[kOffFlag], 1u);
         return;
     }
-    unsigned e = ind[0] + (unsigned)mp.nel[0] * (ind[1] + (unsigned)mp.nel[1] * ind[2]);
+    unsigned e = (unsigned)ind[0] + (unsigned)mp.nel[0] * ((unsigned)ind[1] + (unsigned)mp.nel[1] * (unsigned)ind[2]);
     s[kOffCell + p] = e;
     atomicAdd(&s[kOffCount + e], 1u);
 }
@@ -219,6 +203,7 @@ extern "C" int uwgpu_bin_and_map_noalloc(int32_t dim, const int32_t nel[3], cons
         ne *= mp.nel[d];
     }
     if (n > kMaxPoints || ne > kMaxElements) return UWGPU_ERR_TOO_LARGE;
+    for (int d = 0; d < 3; ++d) mp.ax[d] = uwg::axis_map(mp.min[d], mp.max[d], mp.nel[d]);
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return UWGPU_ERR_CUDA;
     uint32_t* s = scratch_address(dev);

@@ -16,15 +16,20 @@
 // GPU design.  On the affine elements of a regular mesh every product of shape-function
 // derivatives is a polynomial of degree <= 2 per axis in the local coordinates, so
 //   K_e = sum over 3^dim moments mu_abc = sum_p w eta_p xi^a eta^b zeta^c of fixed matrices.
-// One thread owns one element: it streams the element's points (slot order, SoA) once,
-// evaluates the rheology, accumulates the 27 (3D) / 9 (2D) moments in FP64 registers, then
-// contracts them axis by axis into the 300 (3D) / 36 (2D) distinct entries of K_e.  This
-// needs ~50 FP64 operations per point instead of the ~1000 of the per-point B^T D B loop,
-// which matters on a part whose FP64 rate is 1/58 of its FP32 rate.  K_e, f_e, G_e are
-// written entry-major ([entry][element]) so a warp's stores coalesce.
+// A block owns 32 consecutive elements.  Four lanes share an element's points (slot order, SoA): each
+// evaluates the rheology of every fourth point and accumulates all 27 + 8 (3D) / 9 + 4 (2D) moments in FP64
+// registers; a reduce-scatter over the four lanes leaves them in shared memory.  Then the lanes are the 32
+// elements and the four warps share the contraction, axis by axis, into the 63 (10) pair tables and from
+// them the 300 (36) distinct entries of K_e, written entry-major ([entry][element], whole lines per warp).
+// FP64 instructions are what counts (64 cycles per warp and scheduler): about 50 per point of a viscous 3D
+// material and 650 per element here, where one thread per element with generic products took 85 and 4,100
+// and left most of the chip idle on small meshes (32^3 mesh, 27 points: 1,740 us before).
 #include <cuda_fp16.h>
 
+#include <cstring>
+
 #include "internal.cuh"
+#include "locate.cuh"
 #include "tc.cuh"
 
 namespace uwg {
@@ -41,7 +46,9 @@ struct AssemblyArgs {
     const double* seta_in;   // optional
     const double* srho_in;   // optional
     const uwgpu_material* mats;
+    const MaterialInfo* info;   // per material, from k_material_info
     int nmat;
+    const double* tab[3];       // per axis x0[nel], h[nel], 1/h[nel] (binning.cu)
     const double* temperature;  // nodal or null
     const double* u;            // nodal SoA [d][node] or null
     const double* p;            // per element or null
@@ -191,13 +198,46 @@ __device__ inline void sym_eigenvalues(const double* t, int dim, double* ev) {
             }
 }
 
+// What a material's laws need that is the same at every point: formed once per uwgpu_materials_set, not per
+// point (the angle functions of Drucker-Prager cost more than the rest of its evaluation).
+__global__ void k_material_info(int n, const uwgpu_material* __restrict__ mats, MaterialInfo* __restrict__ info) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const uwgpu_material& m = mats[k];
+    MaterialInfo& o = info[k];
+    int needs = 0;
+    for (int l = 0; l < m.n_laws; ++l) {
+        const uwgpu_law& law = m.laws[l];
+        if (law.law == UWGPU_LAW_DRUCKER_PRAGER) {
+            // DruckerPrager.c:251-283: friction and cohesion terms in 2D and in 3D
+            const double phi = atan(law.p[1]);
+            o.dp[l][0][0] = sin(phi);
+            o.dp[l][0][1] = law.p[0] * cos(phi);
+            const double sinphi = sin(phi);
+            const double ood = 1.0 / (sqrt(3.0) * (3.0 - sinphi));
+            o.dp[l][1][0] = 6.0 * sinphi * ood;
+            o.dp[l][1][1] = 6.0 * law.p[0] * cos(phi) * ood;
+        }
+        needs |= law.law == UWGPU_LAW_DRUCKER_PRAGER || law.law == UWGPU_LAW_VON_MISES || law.law == UWGPU_LAW_BYERLEE ||
+                 law.law == UWGPU_LAW_MOHR_COULOMB || law.law == UWGPU_LAW_NON_NEWTONIAN;
+    }
+    o.needs_gradient = needs;
+}
+
+void material_info(Context& c, int n) {
+    c.mat_info.ensure((size_t)n);
+    k_material_info<<<blocks_for(n, 64), 64, 0, c.stream>>>(n, c.mats.p, c.mat_info.p);
+    check_launch("k_material_info");
+}
+
 // Per-point rheology chain.  Every law in scope keeps D isotropic, so the constitutive matrix
 // is carried as its viscosity (D[3][3] in 3D, D[2][2] in 2D).
 template <int DIM>
-__device__ __forceinline__ double run_rheology(const uwgpu_material& m, const double* N, const double* Tn,
-                                               bool hasT, const double* xg, double ymax, double point_eta,
+__device__ __forceinline__ double run_rheology(const uwgpu_material& m, const MaterialInfo& info, double T,
+                                               const double* xg, double ymax, double point_eta,
                                                const double (*L)[3], double pressure, int prev, double pfw,
                                                double* pfw_incr, double* derivs = nullptr, bool jacobian = false) {
+    // T: temperature at the point (0 without a field); L: velocity gradient (used where info.needs_gradient)
     const double yglobal = xg[1];
     double eta = 0.0;
     // derivs: the viscosity derivatives of the Newton form (9 entries; zeroed with every
@@ -227,11 +267,6 @@ __device__ __forceinline__ double run_rheology(const uwgpu_material& m, const do
             set_visc(law.p[0]);
             break;
         case UWGPU_LAW_ARRHENIUS: {
-            double T = 0.0;
-            if (hasT) {
-#pragma unroll
-                for (int a = 0; a < (1 << DIM); ++a) T += N[a] * Tn[a];
-            }
             if (law.p[2] > (0.0 + 1e-12)) {
                 double depth = ymax - yglobal;
                 set_visc(law.p[0] * exp((law.p[1] + law.p[2] * depth) / (T + law.p[3])));
@@ -240,15 +275,9 @@ __device__ __forceinline__ double run_rheology(const uwgpu_material& m, const do
             }
             break;
         }
-        case UWGPU_LAW_FRANK_KAMENETSKII: {
-            double T = 0.0;
-            if (hasT) {
-#pragma unroll
-                for (int a = 0; a < (1 << DIM); ++a) T += N[a] * Tn[a];
-            }
+        case UWGPU_LAW_FRANK_KAMENETSKII:
             set_visc(law.p[0] * exp(-law.p[1] * T));
             break;
-        }
         case UWGPU_LAW_VISCOSITY_LIMITER: {
             double v = eta;
             if (v > law.p[0]) v = law.p[0];
@@ -273,17 +302,7 @@ __device__ __forceinline__ double run_rheology(const uwgpu_material& m, const do
                 inv = 0.5 * (s0 * s0 + s1 * s1) + s2 * s2;
             }
             double ind = sqrt(inv);
-            double phi = atan(law.p[1]);
-            double dpFric, dpCoh;
-            if (DIM == 3) {
-                double sinphi = sin(phi);
-                double ood = 1.0 / (sqrt(3.0) * (3.0 - sinphi));
-                dpFric = 6.0 * sinphi * ood;
-                dpCoh = 6.0 * law.p[0] * cos(phi) * ood;
-            } else {
-                dpCoh = law.p[0] * cos(phi);
-                dpFric = sin(phi);
-            }
+            const double dpFric = info.dp[l][DIM - 2][0], dpCoh = info.dp[l][DIM - 2][1];
             double crit = dpFric * pressure + dpCoh;
             if (crit < law.p[2]) crit = law.p[2];
             if (crit < ind) {
@@ -445,14 +464,11 @@ __device__ __forceinline__ double run_rheology(const uwgpu_material& m, const do
     return eta;
 }
 
-// Coefficients of (1 + s_i x)(1 + s_j x) in the monomials 1, x, x^2, by pair type:
-// type 0: s_i = s_j = +1, type 1: s_i = s_j = -1, type 2: s_i != s_j.
-__device__ __constant__ double kQ[3][3] = {{1.0, 2.0, 1.0}, {1.0, -2.0, 1.0}, {1.0, 0.0, -1.0}};
-// Coefficients of (1 + s x) in 1, x by type: 0: s = +1, 1: s = -1.
-__device__ __constant__ double kL[2][2] = {{1.0, 1.0}, {1.0, -1.0}};
-
-__device__ __forceinline__ int qtype(int si, int sj) { return si == sj ? (si > 0 ? 0 : 1) : 2; }
-__device__ __forceinline__ int ltype(int s) { return s > 0 ? 0 : 1; }
+// Pair type of two nodes along an axis, for (1 + s_i x)(1 + s_j x) in the monomials 1, x, x^2:
+// type 0: s_i = s_j = +1 (1, 2, 1), type 1: s_i = s_j = -1 (1, -2, 1), type 2: s_i != s_j (1, 0, -1); and type
+// of 1 + s x: 0: s = +1, 1: s = -1.
+__host__ __device__ constexpr int qtype(int si, int sj) { return si == sj ? (si > 0 ? 0 : 1) : 2; }
+__host__ __device__ constexpr int ltype(int s) { return s > 0 ? 0 : 1; }
 
 // The 63 pair tables of a 3D element: same-axis tables Dkk[t1][t2] (the node-pair types of the two
 // other axes) and mixed-axis tables Mkl[t_k][t_l][t_other], each an integer combination of the 27
@@ -486,51 +502,6 @@ __host__ __device__ inline int table_coefficient(int q, int m) {
     else { u = b; v = c; o = a; }                  // yz
     if (u > 1 || v > 1) return 0;
     return L[ta][u] * L[tb][v] * Q[to][o];
-}
-
-__device__ __forceinline__ void tables_from_moments(const double* mu, Tables3& T) {
-#pragma unroll
-    for (int t1 = 0; t1 < 3; ++t1)
-#pragma unroll
-        for (int t2 = 0; t2 < 3; ++t2) {
-            double sx = 0.0, sy = 0.0, sz = 0.0;
-#pragma unroll
-            for (int u = 0; u < 3; ++u)
-#pragma unroll
-                for (int v = 0; v < 3; ++v) {
-                    double q = kQ[t1][u] * kQ[t2][v];
-                    sx += q * mu[0 * 9 + u * 3 + v];   // axes y (u), z (v)
-                    sy += q * mu[u * 9 + 0 * 3 + v];   // axes x (u), z (v)
-                    sz += q * mu[u * 9 + v * 3 + 0];   // axes x (u), y (v)
-                }
-            T.Dxx[t1][t2] = sx;
-            T.Dyy[t1][t2] = sy;
-            T.Dzz[t1][t2] = sz;
-        }
-#pragma unroll
-    for (int ta = 0; ta < 2; ++ta)
-#pragma unroll
-        for (int tb = 0; tb < 2; ++tb)
-#pragma unroll
-            for (int to = 0; to < 3; ++to) {
-                double sxy = 0.0, sxz = 0.0, syz = 0.0;
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
-#pragma unroll
-                    for (int v = 0; v < 2; ++v) {
-                        double l2 = kL[ta][u] * kL[tb][v];
-#pragma unroll
-                        for (int o = 0; o < 3; ++o) {
-                            double q = l2 * kQ[to][o];
-                            sxy += q * mu[u * 9 + v * 3 + o];   // x^u y^v z^o
-                            sxz += q * mu[u * 9 + o * 3 + v];   // x^u z^v y^o
-                            syz += q * mu[o * 9 + u * 3 + v];   // y^u z^v x^o
-                        }
-                    }
-                T.Mxy[ta][tb][to] = sxy;
-                T.Mxz[ta][tb][to] = sxz;
-                T.Myz[ta][tb][to] = syz;
-            }
 }
 
 // Packed K_e (entry-major) of element e from its tables; diag receives the 24 diagonal entries.
@@ -578,284 +549,402 @@ __device__ __forceinline__ void ke_from_tables(const Tables3& T, double detJ, co
         }
 }
 
+// Node pairs (i, j), i <= j, dealt to the four warps of a block: every warp gets as many diagonal pairs (whose
+// entries also enter S_e) as any other.
 template <int DIM>
-__global__ void __launch_bounds__(128) k_assemble(AssemblyArgs A) {
-    constexpr int NEN = 1 << DIM;
-    constexpr int ND = NEN * DIM;
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= A.ne) return;
-    int64_t ie = e % A.nel[0];
-    int64_t je = (e / A.nel[0]) % A.nel[1];
-    int64_t ke = DIM == 3 ? e / ((int64_t)A.nel[0] * A.nel[1]) : 0;
-    int64_t idx[3] = {ie, je, ke};
-    double x0[3], h[3];
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-        x0[d] = node_coord_1d(idx[d], A.nel[d], A.min[d], A.max[d]);
-        h[d] = node_coord_1d(idx[d] + 1, A.nel[d], A.min[d], A.max[d]) - x0[d];
+struct PairList {
+    static constexpr int kNen = 1 << DIM, kMax = (kNen * (kNen + 1) / 2 + 3) / 4 + 1;
+    int i[4][kMax] = {}, j[4][kMax] = {}, n[4] = {};
+    constexpr PairList() {
+        for (int a = 0; a < kNen; ++a) add(a % 4, a, a);
+        int next = 0;
+        for (int a = 0; a < kNen; ++a)
+            for (int b = a + 1; b < kNen; ++b) add(next++ % 4, a, b);
     }
-    // element nodes (CartesianGenerator incidence order, x fastest)
-    int64_t base = ie + A.nnx * (je + A.nny * ke);
-    int64_t inc[NEN];
-#pragma unroll
-    for (int a = 0; a < NEN; ++a)
-        inc[a] = base + (a & 1) + ((a >> 1) & 1) * A.nnx + (DIM == 3 ? ((a >> 2) & 1) * A.nnx * A.nny : 0);
-    double Tn[NEN];
-    bool hasT = A.temperature != nullptr;
-#pragma unroll
-    for (int a = 0; a < NEN; ++a) Tn[a] = hasT ? A.temperature[inc[a]] : 0.0;
-    bool needL = A.u != nullptr && A.previous_solution;
-    double un[DIM][NEN];
-    if (needL) {
-#pragma unroll
-        for (int d = 0; d < DIM; ++d)
-#pragma unroll
-            for (int a = 0; a < NEN; ++a) un[d][a] = A.u[(int64_t)d * A.nn + inc[a]];
+    constexpr void add(int w, int a, int b) {
+        i[w][n[w]] = a;
+        j[w][n[w]] = b;
+        ++n[w];
     }
-    double pressure = A.p ? A.p[e] : 0.0;
+};
 
-    uint32_t beg = A.offsets[e], end = A.offsets[e + 1];
-    uint32_t cnt = end - beg;
-    if (cnt == 0) atomicOr(A.flags, 1u);
-    const double cellVolume = DIM == 3 ? 8.0 : 4.0;
-    double w = cellVolume / (double)cnt;
+constexpr int kAsEl = 32, kAsPitch = 33;   // elements per block, and the pitch of per-element shared arrays
 
-    constexpr int NM = DIM == 3 ? 27 : 9;
-    constexpr int NF = NEN;
-    double mu[NM];
-    double phi[NF];
-#pragma unroll
-    for (int i = 0; i < NM; ++i) mu[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < NF; ++i) phi[i] = 0.0;
+template <int DIM>
+struct AssembleSmem {
+    static constexpr int NEN = 1 << DIM, NM = DIM == 3 ? 27 : 9, NT = DIM == 3 ? 63 : 10;
+    double mom[NM + NEN][kAsPitch];       // moments of viscosity, then of density
+    union {
+        double field[(DIM + 1) * NEN][kAsPitch];   // monomial coefficients of velocity and temperature
+        double tab[NT][kAsPitch];                  // pair tables, scaled
+    };
+    double s[4][kAsPitch];
+};
 
-    for (uint32_t s = beg; s < end; ++s) {
-        double xi[3];
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) xi[d] = A.sxi[(int64_t)d * A.nslots + s];
-        if (DIM == 2) xi[2] = 0.0;
-        int mi = A.smat[s];
-        if (mi < 0 || mi >= A.nmat) {
-            atomicOr(A.flags, 2u);
-            mi = 0;
-        }
-        const uwgpu_material& m = A.mats[mi];
-        // shape functions at xi (TrilinearElementType.c:249-263 / BilinearElementType.c:212-220)
-        double N[NEN];
-#pragma unroll
-        for (int a = 0; a < NEN; ++a) {
-            double v = DIM == 3 ? 0.125 : 0.25;
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) v *= ((a >> d) & 1) ? (1.0 + xi[d]) : (1.0 - xi[d]);
-            N[a] = v;
-        }
-        double L[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        if (needL) {
-            // velocity gradient L[i][j] = du_i/dx_j from the global derivatives at xi
-#pragma unroll
-            for (int a = 0; a < NEN; ++a) {
-                double gx[3];
-#pragma unroll
-                for (int d = 0; d < DIM; ++d) {
-                    double v = (2.0 / h[d]) * (DIM == 3 ? 0.125 : 0.25) * (((a >> d) & 1) ? 1.0 : -1.0);
-#pragma unroll
-                    for (int q = 0; q < DIM; ++q)
-                        if (q != d) v *= ((a >> q) & 1) ? (1.0 + xi[q]) : (1.0 - xi[q]);
-                    gx[d] = v;
-                }
-#pragma unroll
-                for (int i = 0; i < DIM; ++i)
-#pragma unroll
-                    for (int j = 0; j < DIM; ++j) L[i][j] += gx[j] * un[i][a];
-            }
-        }
-        // global coordinate of the point (FeMesh_CoordLocalToGlobal on the affine element)
-        double xg[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) xg[d] = x0[d] + 0.5 * h[d] * (xi[d] + 1.0);
-        double peta = A.seta_in ? A.seta_in[s] : 0.0;
-        const uint32_t pidx = A.perm[s];
-        double eta = run_rheology<DIM>(m, N, Tn, hasT, xg, A.max[1], peta, L, pressure, A.previous_solution,
-                                       A.pfw ? A.pfw[pidx] : 0.0, A.pfw_incr ? A.pfw_incr + pidx : nullptr);
-        if (A.eta_out) A.eta_out[s] = eta;
-        double rho0 = A.srho_in ? A.srho_in[s] : m.density;
-        double T = 0.0;
-        if (hasT && m.alpha != 0.0) {
-#pragma unroll
-            for (int a = 0; a < NEN; ++a) T += N[a] * Tn[a];
-        }
-        double rho = rho0 * (1.0 - m.alpha * (T - m.ref_temp));
+// (a, b, c) -> (a + 2 b + c, a - 2 b + c, a - c): the three pair types of one axis
+__device__ __forceinline__ void pair_types(double& a, double& b, double& c) {
+    const double s = a + c, d = a - c;
+    a = fma(2.0, b, s);
+    b = fma(-2.0, b, s);
+    c = d;
+}
 
-        const double ws = A.sw ? A.sw[s] : w;
-        double c = ws * eta;
-        double r = ws * rho;
-        if (DIM == 3) {
-            double x1 = xi[0], y1 = xi[1], z1 = xi[2];
-            double x2 = x1 * x1;
-            double cz0 = c, cz1 = c * z1, cz2 = cz1 * z1;
-            double cyz[3][3];
-            cyz[0][0] = cz0;
-            cyz[0][1] = cz1;
-            cyz[0][2] = cz2;
-            cyz[1][0] = cz0 * y1;
-            cyz[1][1] = cz1 * y1;
-            cyz[1][2] = cz2 * y1;
-            cyz[2][0] = cyz[1][0] * y1;
-            cyz[2][1] = cyz[1][1] * y1;
-            cyz[2][2] = cyz[1][2] * y1;
-#pragma unroll
-            for (int b = 0; b < 3; ++b)
-#pragma unroll
-                for (int cc = 0; cc < 3; ++cc) {
-                    double v = cyz[b][cc];
-                    mu[0 * 9 + b * 3 + cc] += v;
-                    mu[1 * 9 + b * 3 + cc] = fma(x1, v, mu[1 * 9 + b * 3 + cc]);
-                    mu[2 * 9 + b * 3 + cc] = fma(x2, v, mu[2 * 9 + b * 3 + cc]);
-                }
-            double rz = r * z1, ry = r * y1, ryz = ry * z1;
-            phi[0] += r;
-            phi[1] = fma(x1, r, phi[1]);
-            phi[2] += ry;
-            phi[3] = fma(x1, ry, phi[3]);
-            phi[4] += rz;
-            phi[5] = fma(x1, rz, phi[5]);
-            phi[6] += ryz;
-            phi[7] = fma(x1, ryz, phi[7]);
-        } else {
-            double x1 = xi[0], y1 = xi[1];
-            double x2 = x1 * x1;
-            double cy0 = c, cy1 = c * y1, cy2 = cy1 * y1;
-            double cy[3] = {cy0, cy1, cy2};
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                mu[0 * 3 + b] += cy[b];
-                mu[1 * 3 + b] = fma(x1, cy[b], mu[1 * 3 + b]);
-                mu[2 * 3 + b] = fma(x2, cy[b], mu[2 * 3 + b]);
-            }
-            double ry = r * y1;
-            phi[0] += r;
-            phi[1] = fma(x1, r, phi[1]);
-            phi[2] += ry;
-            phi[3] = fma(x1, ry, phi[3]);
-        }
-    }
-
-    // ---- contraction of the moments into K_e ----
-    // detJ of the affine element and derivative scales (ElementType.c:354-495 reduces to these)
-    double detJ = DIM == 3 ? (0.5 * h[0]) * (0.5 * h[1]) * (0.5 * h[2]) : (0.5 * h[0]) * (0.5 * h[1]);
-    double g[3];
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) g[d] = 2.0 / h[d];
-    const double inv64 = DIM == 3 ? 1.0 / 64.0 : 1.0 / 16.0;
-
-    if (DIM == 3) {
-        const int64_t ne = A.ne;
-        double diag[ND];
-        if (A.mom) {
-            // moments out; K_e and S_e come from the tensor-core contraction (k_contract_tc)
-#pragma unroll
-            for (int m = 0; m < NM; ++m) A.mom[(int64_t)m * ne + e] = mu[m];
-        } else {
-            Tables3 T;
-            tables_from_moments(mu, T);
-            ke_from_tables(T, detJ, g, e, ne, A.Ke, diag);
-        }
-        // G_e: integral of -dN_a/dx_d over the element (exact for the 2x2x2 Gauss rule)
-        double s = 0.0;
-#pragma unroll
-        for (int a = 0; a < NEN; ++a)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const double G = ge_entry(h, a, d);
-                A.Ge[(int64_t)(a * 3 + d) * ne + e] = G;
-                if (!A.mom) s += G * (G / diag[a * 3 + d]);
-            }
-        if (!A.mom) A.Se[e] = s;
-        // f_e: -g detJ sum_p w rho N_a on the vertical component
-        double fs = -A.gravity * detJ * 0.125;
-#pragma unroll
-        for (int a = 0; a < NEN; ++a) {
-            double sx = (a & 1) ? 1.0 : -1.0, sy = ((a >> 1) & 1) ? 1.0 : -1.0, sz = ((a >> 2) & 1) ? 1.0 : -1.0;
-            double v = phi[0] + sx * phi[1] + sy * phi[2] + sx * sy * phi[3] + sz * phi[4] + sx * sz * phi[5] +
-                       sy * sz * phi[6] + sx * sy * sz * phi[7];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) A.fe[(int64_t)(a * 3 + d) * ne + e] = (d == A.vert_axis) ? fs * v : 0.0;
-        }
-    } else {
-        double Dxx[3], Dyy[3];
+// The pair tables of element `lane`, group `grp` of six in 3D (Dxx, Dyy, Dzz, Mxy, Mxz, Myz), all in 2D;
+// scaled by detJ g_k g_l / 4^dim
+template <int DIM>
+__device__ __forceinline__ void form_tables(AssembleSmem<DIM>& S, int lane, int grp, double detJ, const double* g) {
+    auto mu = [&](int m) { return S.mom[m][lane]; };
+    if (DIM == 2) {
+        double x[3] = {mu(0), mu(1), mu(2)}, y[3] = {mu(0), mu(3), mu(6)};
+        const double c00 = mu(0), c01 = mu(1), c10 = mu(3), c11 = mu(4);
+        pair_types(x[0], x[1], x[2]);
+        pair_types(y[0], y[1], y[2]);
+        const double sxx = detJ * g[0] * g[0] * (1.0 / 16.0), syy = detJ * g[1] * g[1] * (1.0 / 16.0),
+                     sxy = detJ * g[0] * g[1] * (1.0 / 16.0);
 #pragma unroll
         for (int t = 0; t < 3; ++t) {
-            double sx = 0.0, sy = 0.0;
-#pragma unroll
-            for (int u = 0; u < 3; ++u) {
-                sx += kQ[t][u] * mu[0 * 3 + u];
-                sy += kQ[t][u] * mu[u * 3 + 0];
-            }
-            Dxx[t] = sx;
-            Dyy[t] = sy;
+            S.tab[t][lane] = sxx * x[t];
+            S.tab[3 + t][lane] = syy * y[t];
         }
-        double Mxy[2][2];
+        const double p = c00 + c01, q = c10 + c11, r = c00 - c01, w = c10 - c11;
+        S.tab[6][lane] = sxy * (p + q);    // [ta = +][tb = +]
+        S.tab[7][lane] = sxy * (r + w);    // [+][-]
+        S.tab[8][lane] = sxy * (p - q);    // [-][+]
+        S.tab[9][lane] = sxy * (r - w);    // [-][-]
+        return;
+    }
+    if (grp < 3) {
+        double m[3][3];
 #pragma unroll
-        for (int ta = 0; ta < 2; ++ta)
+        for (int u = 0; u < 3; ++u)
 #pragma unroll
-            for (int tb = 0; tb < 2; ++tb) {
-                double v = 0.0;
+            for (int v = 0; v < 3; ++v) m[u][v] = mu(grp == 0 ? u * 3 + v : grp == 1 ? u * 9 + v : u * 9 + v * 3);
 #pragma unroll
-                for (int u = 0; u < 2; ++u)
+        for (int v = 0; v < 3; ++v) pair_types(m[0][v], m[1][v], m[2][v]);
+        const double gg = grp == 0 ? g[0] : grp == 1 ? g[1] : g[2];
+        const double sc = detJ * gg * gg * (1.0 / 64.0);
 #pragma unroll
-                    for (int q = 0; q < 2; ++q) v += kL[ta][u] * kL[tb][q] * mu[u * 3 + q];
-                Mxy[ta][tb] = v;
+        for (int u = 0; u < 3; ++u) {
+            pair_types(m[u][0], m[u][1], m[u][2]);
+#pragma unroll
+            for (int v = 0; v < 3; ++v) S.tab[grp * 9 + u * 3 + v][lane] = sc * m[u][v];
+        }
+    } else {
+        // powers u, v <= 1 of the pair's axes and o of the other: xy (9u + 3v + o), xz (9u + v + 3o), yz (3u + v + 9o)
+        const int pu = grp == 5 ? 3 : 9, pv = grp == 3 ? 3 : 1, po = grp == 3 ? 1 : grp == 4 ? 3 : 9;
+        const double sc = detJ * (grp == 5 ? g[1] : g[0]) * (grp == 3 ? g[1] : g[2]) * (1.0 / 64.0);
+        double m[2][2][3];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+#pragma unroll
+                for (int o = 0; o < 3; ++o) m[u][v][o] = mu(u * pu + v * pv + o * po);
+                pair_types(m[u][v][0], m[u][v][1], m[u][v][2]);
             }
-        auto Mkl = [&](int k, int l, int i, int j) -> double {
-            int si[2] = {((i & 1) << 1) - 1, (((i >> 1) & 1) << 1) - 1};
-            int sj[2] = {((j & 1) << 1) - 1, (((j >> 1) & 1) << 1) - 1};
-            double sc = detJ * g[k] * g[l] * inv64 * (double)(si[k] * sj[l]);
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+            const double p = m[0][0][o] + m[0][1][o], q = m[1][0][o] + m[1][1][o];
+            const double r = m[0][0][o] - m[0][1][o], w = m[1][0][o] - m[1][1][o];
+            const int b = 27 + (grp - 3) * 12 + o;
+            S.tab[b][lane] = sc * (p + q);
+            S.tab[b + 3][lane] = sc * (r + w);
+            S.tab[b + 6][lane] = sc * (p - q);
+            S.tab[b + 9][lane] = sc * (r - w);
+        }
+    }
+}
+
+// K_e entries of warp W's node pairs of element e (lane), and its part of S_e
+template <int DIM, int W>
+__device__ __forceinline__ void form_entries(AssembleSmem<DIM>& S, int lane, const double* h, int64_t e, int64_t ne,
+                                             double* __restrict__ Ke, bool live) {
+    constexpr PairList<DIM> P{};
+    constexpr int ND = (1 << DIM) * DIM;
+    double part = 0.0;
+#pragma unroll
+    for (int t = 0; t < P.n[W]; ++t) {
+        const int i = P.i[W][t], j = P.j[W][t];
+        // M_kl[i][j]: derivative along k on node i, along l on node j
+        auto M = [&](int k, int l) -> double {
+            int si[3] = {(i & 1) * 2 - 1, ((i >> 1) & 1) * 2 - 1, ((i >> 2) & 1) * 2 - 1};
+            int sj[3] = {(j & 1) * 2 - 1, ((j >> 1) & 1) * 2 - 1, ((j >> 2) & 1) * 2 - 1};
+            const int sign = si[k] * sj[l];
+            int q;
             if (k == l) {
-                if (k == 0) return sc * Dxx[qtype(si[1], sj[1])];
-                return sc * Dyy[qtype(si[0], sj[0])];
+                if (DIM == 3) {
+                    const int a = k == 0 ? 1 : 0, b = k == 2 ? 1 : 2;   // the other two axes
+                    q = k * 9 + qtype(si[a], sj[a]) * 3 + qtype(si[b], sj[b]);
+                } else {
+                    q = k * 3 + qtype(si[1 - k], sj[1 - k]);
+                }
+            } else {
+                // the tables hold k < l; M_lk[i][j] = M_kl[j][i]
+                const int a = k < l ? k : l, b = k < l ? l : k;
+                const int ta = k < l ? ltype(sj[a]) : ltype(si[a]), tb = k < l ? ltype(si[b]) : ltype(sj[b]);
+                if (DIM == 3) {
+                    const int o = 3 - a - b;
+                    q = 27 + (a + b - 1) * 12 + ta * 6 + tb * 3 + qtype(si[o], sj[o]);
+                } else {
+                    q = 6 + ta * 2 + tb;
+                }
             }
-            if (k > l) {
-                for (int q = 0; q < 2; ++q) { int t = si[q]; si[q] = sj[q]; sj[q] = t; }
-            }
-            return sc * Mxy[ltype(sj[0])][ltype(si[1])];
+            return sign > 0 ? S.tab[q][lane] : -S.tab[q][lane];
         };
-        const int64_t ne = A.ne;
-        double diag[ND];
+        double d[DIM], tr = 0.0;
 #pragma unroll
-        for (int i = 0; i < NEN; ++i)
-#pragma unroll
-            for (int j = i; j < NEN; ++j) {
-                double tr = Mkl(0, 0, i, j) + Mkl(1, 1, i, j);
-#pragma unroll
-                for (int al = 0; al < 2; ++al)
-#pragma unroll
-                    for (int be = 0; be < 2; ++be) {
-                        int r = i * 2 + al, cix = j * 2 + be;
-                        if (r > cix) continue;
-                        double v = Mkl(be, al, i, j) + (al == be ? tr : 0.0);
-                        A.Ke[(int64_t)packed_index(ND, r, cix) * ne + e] = v;
-                        if (r == cix) diag[r] = v;
-                    }
-            }
-        double s = 0.0;
-#pragma unroll
-        for (int a = 0; a < NEN; ++a)
-#pragma unroll
-            for (int d = 0; d < 2; ++d) {
-                double sa = ((a >> d) & 1) ? 1.0 : -1.0;
-                double G = -sa * h[1 - d] * 0.5;
-                A.Ge[(int64_t)(a * 2 + d) * ne + e] = G;
-                s += G * (G / diag[a * 2 + d]);
-            }
-        A.Se[e] = s;
-        double fs = -A.gravity * detJ * 0.25;
-#pragma unroll
-        for (int a = 0; a < NEN; ++a) {
-            double sx = (a & 1) ? 1.0 : -1.0, sy = ((a >> 1) & 1) ? 1.0 : -1.0;
-            double v = phi[0] + sx * phi[1] + sy * phi[2] + sx * sy * phi[3];
-#pragma unroll
-            for (int d = 0; d < 2; ++d) A.fe[(int64_t)(a * 2 + d) * ne + e] = (d == A.vert_axis) ? fs * v : 0.0;
+        for (int k = 0; k < DIM; ++k) {
+            d[k] = M(k, k);
+            tr = k == 0 ? d[0] : tr + d[k];
         }
+#pragma unroll
+        for (int al = 0; al < DIM; ++al)
+#pragma unroll
+            for (int be = 0; be < DIM; ++be) {
+                const int r = i * DIM + al, q = j * DIM + be;
+                if (r > q) continue;
+                // K[(i,al),(j,be)] = delta * tr + M_{be,al}[i][j]
+                const double v = al == be ? d[al] + tr : M(be, al);
+                if (live) Ke[(int64_t)packed_index(ND, r, q) * ne + e] = v;
+                if (r == q) {
+                    // S_e = sum G^2 / K_rr; with G^2 the same for all nodes of a component
+                    double area = 1.0;
+#pragma unroll
+                    for (int o = 0; o < DIM; ++o)
+                        if (o != al) area *= h[o];
+                    const double G = area * (DIM == 3 ? 0.25 : 0.5);
+                    part += G * (G / v);
+                }
+            }
+    }
+    S.s[W][lane] = part;
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(128, 3) k_assemble(const __grid_constant__ AssemblyArgs A) {
+    constexpr int NEN = 1 << DIM, NM = DIM == 3 ? 27 : 9, NS = NM + NEN;
+    __shared__ AssembleSmem<DIM> S;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t e0 = (int64_t)blockIdx.x * kAsEl;
+    // geometry and nodes of element e
+    auto layers = [&](int64_t e, int idx[3]) {
+        const unsigned nx = (unsigned)A.nel[0], q = (unsigned)e / nx;
+        idx[0] = (int)((unsigned)e - q * nx);
+        idx[1] = DIM == 3 ? (int)(q % (unsigned)A.nel[1]) : (int)q;
+        idx[2] = DIM == 3 ? (int)(q / (unsigned)A.nel[1]) : 0;
+    };
+    const bool hasT = A.temperature != nullptr;
+    const bool hasU = A.u != nullptr && A.previous_solution;
+    if (hasT || hasU) {
+        // the fields as polynomials of the local coordinates: 2^dim monomial coefficients per component
+        // (one thread per element and component), so a value or derivative at a point is a few FMAs
+        const int64_t e = e0 + lane;
+        for (int f = warp; f < DIM + 1; f += 4) {
+            if (f < DIM ? !hasU : !hasT) continue;
+            double v[NEN];
+            if (e < A.ne) {
+                int idx[3];
+                layers(e, idx);
+                const int64_t base = idx[0] + A.nnx * (idx[1] + A.nny * (int64_t)idx[2]);
+                const double* src = f < DIM ? A.u + (int64_t)f * A.nn : A.temperature;
+#pragma unroll
+                for (int a = 0; a < NEN; ++a)
+                    v[a] = src[base + (a & 1) + ((a >> 1) & 1) * A.nnx + (DIM == 3 ? ((a >> 2) & 1) * A.nnx * A.nny : 0)];
+            } else {
+#pragma unroll
+                for (int a = 0; a < NEN; ++a) v[a] = 0.0;
+            }
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+#pragma unroll
+                for (int a = 0; a < NEN; ++a)
+                    if (!((a >> d) & 1)) {
+                        const double lo = v[a], hi = v[a | (1 << d)];
+                        v[a] = 0.5 * (lo + hi);
+                        v[a | (1 << d)] = 0.5 * (hi - lo);
+                    }
+#pragma unroll
+            for (int a = 0; a < NEN; ++a) S.field[f * NEN + a][lane] = v[a];
+        }
+        __syncthreads();
+    }
+    // ---- points: lanes 4 el .. 4 el + 3 of the block's threads share element el ----
+    {
+        const int el = tid >> 2, part = tid & 3;
+        const int64_t e = e0 + el;
+        double m[NS + 1];
+#pragma unroll
+        for (int k = 0; k <= NS; ++k) m[k] = 0.0;
+        if (e < A.ne) {
+            int idx[3];
+            layers(e, idx);
+            const uint32_t beg = A.offsets[e], end = A.offsets[e + 1];
+            if (end == beg && part == 0) atomicOr(A.flags, 1u);
+            const double w = (DIM == 3 ? 8.0 : 4.0) / (double)(end - beg);
+            const double pressure = A.p ? A.p[e] : 0.0;
+            for (uint32_t s = beg + part; s < end; s += 4) {
+                double xi[3];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) xi[d] = A.sxi[(int64_t)d * A.nslots + s];
+                if (DIM == 2) xi[2] = 0.0;
+                int mi = A.smat[s];
+                if (mi < 0 || mi >= A.nmat) {
+                    atomicOr(A.flags, 2u);
+                    mi = 0;
+                }
+                const uwgpu_material& mat = A.mats[mi];
+                const MaterialInfo& info = A.info[mi];
+                const double xy = xi[0] * xi[1], xz = DIM == 3 ? xi[0] * xi[2] : 0.0, yz = DIM == 3 ? xi[1] * xi[2] : 0.0;
+                double T = 0.0;
+                if (hasT) {
+                    auto c = [&](int a) { return S.field[DIM * NEN + a][el]; };
+                    T = fma(c(3), xy, fma(c(2), xi[1], fma(c(1), xi[0], c(0))));
+                    if (DIM == 3) T = fma(c(7), xy * xi[2], fma(c(6), yz, fma(c(5), xz, fma(c(4), xi[2], T))));
+                }
+                double L[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+                if (hasU && info.needs_gradient) {
+                    // velocity gradient L[i][j] = du_i/dx_j = 2/h_j du_i/dxi_j
+#pragma unroll
+                    for (int i = 0; i < DIM; ++i) {
+                        auto c = [&](int a) { return S.field[i * NEN + a][el]; };
+                        double dx = fma(c(3), xi[1], c(1)), dy = fma(c(3), xi[0], c(2));
+                        if (DIM == 3) {
+                            dx = fma(c(7), yz, fma(c(5), xi[2], dx));
+                            dy = fma(c(7), xz, fma(c(6), xi[2], dy));
+                            L[i][2] = fma(c(7), xy, fma(c(6), xi[1], fma(c(5), xi[0], c(4))));
+                        }
+                        L[i][0] = dx;
+                        L[i][1] = dy;
+                    }
+#pragma unroll
+                    for (int j = 0; j < DIM; ++j) {
+                        const double g = 2.0 * __ldg(A.tab[j] + 2 * A.nel[j] + idx[j]);
+#pragma unroll
+                        for (int i = 0; i < DIM; ++i) L[i][j] *= g;
+                    }
+                }
+                // global coordinate of the point (FeMesh_CoordLocalToGlobal on the affine element)
+                double xg[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+                for (int d = 0; d < DIM; ++d)
+                    xg[d] = __ldg(A.tab[d] + idx[d]) + 0.5 * __ldg(A.tab[d] + A.nel[d] + idx[d]) * (xi[d] + 1.0);
+                const double peta = A.seta_in ? A.seta_in[s] : 0.0;
+                const uint32_t pidx = A.pfw ? A.perm[s] : 0u;
+                const double eta = run_rheology<DIM>(mat, info, T, xg, A.max[1], peta, L, pressure, A.previous_solution,
+                                                     A.pfw ? A.pfw[pidx] : 0.0, A.pfw_incr ? A.pfw_incr + pidx : nullptr);
+                if (A.eta_out) A.eta_out[s] = eta;
+                double rho = A.srho_in ? A.srho_in[s] : mat.density;
+                if (mat.alpha != 0.0) rho = rho * (1.0 - mat.alpha * (T - mat.ref_temp));
+                const double ws = A.sw ? A.sw[s] : w;
+                const double c = ws * eta, r = ws * rho, x1 = xi[0], x2 = x1 * x1;
+                double cy[3][3];   // c y^b z^c (2D: c y^b in the first column)
+                cy[0][0] = c;
+                cy[0][1] = c * xi[2];
+                cy[0][2] = cy[0][1] * xi[2];
+#pragma unroll
+                for (int b = 1; b < 3; ++b)
+#pragma unroll
+                    for (int q = 0; q < (DIM == 3 ? 3 : 1); ++q) cy[b][q] = cy[b - 1][q] * xi[1];
+                constexpr int NZ = DIM == 3 ? 3 : 1, NP2 = 3 * NZ;
+#pragma unroll
+                for (int b = 0; b < 3; ++b)
+#pragma unroll
+                    for (int q = 0; q < NZ; ++q) {
+                        const double v = cy[b][q];
+                        m[b * NZ + q] += v;
+                        m[NP2 + b * NZ + q] = fma(x1, v, m[NP2 + b * NZ + q]);
+                        m[2 * NP2 + b * NZ + q] = fma(x2, v, m[2 * NP2 + b * NZ + q]);
+                    }
+                const double ry = r * xi[1];
+                m[NM] += r;
+                m[NM + 1] = fma(x1, r, m[NM + 1]);
+                m[NM + 2] += ry;
+                m[NM + 3] = fma(x1, ry, m[NM + 3]);
+                if (DIM == 3) {
+                    const double rz = r * xi[2], ryz = ry * xi[2];
+                    m[NM + NEN - 4] += rz;
+                    m[NM + NEN - 3] = fma(x1, rz, m[NM + NEN - 3]);
+                    m[NM + NEN - 2] += ryz;
+                    m[NM + NEN - 1] = fma(x1, ryz, m[NM + NEN - 1]);
+                }
+            }
+        }
+        // reduce-scatter over the four lanes: after it, lane `part` holds a quarter of the sums
+        constexpr int H = (NS + 1) / 2, Q = (H + 1) / 2;
+        double a[H + 1], b[Q];
+#pragma unroll
+        for (int k = 0; k < H; ++k) {
+            const double lo = m[k], hi = H + k < NS ? m[H + k] : 0.0;
+            a[k] = (part & 1 ? hi : lo) + __shfl_xor_sync(0xffffffffu, part & 1 ? lo : hi, 1);
+        }
+        a[H] = 0.0;
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            const double lo = a[k], hi = Q + k < H ? a[Q + k] : 0.0;
+            b[k] = (part & 2 ? hi : lo) + __shfl_xor_sync(0xffffffffu, part & 2 ? lo : hi, 2);
+        }
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            const int in_half = (part & 2 ? Q : 0) + k, at = (part & 1 ? H : 0) + in_half;
+            if (in_half < H && at < NS) S.mom[at][el] = b[k];
+        }
+    }
+    __syncthreads();
+    // ---- contraction: lanes are elements ----
+    const int64_t e = e0 + lane, ne = A.ne;
+    const bool live = e < ne;
+    int idx[3];
+    layers(live ? e : 0, idx);
+    double h[3], g[3], detJ = 1.0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        h[d] = __ldg(A.tab[d] + A.nel[d] + idx[d]);
+        g[d] = 2.0 * __ldg(A.tab[d] + 2 * A.nel[d] + idx[d]);
+        detJ = d == 0 ? 0.5 * h[0] : detJ * (0.5 * h[d]);
+    }
+    if (DIM == 3 && A.mom) {
+        // moments out; K_e and S_e come from the tensor-core contraction (k_contract_tc)
+        if (live)
+            for (int k = warp; k < NM; k += 4) A.mom[(int64_t)k * ne + e] = S.mom[k][lane];
+    } else {
+        if (DIM == 3) {
+            for (int grp = warp; grp < 6; grp += 4) form_tables<DIM>(S, lane, grp, detJ, g);
+        } else if (warp == 0) {
+            form_tables<DIM>(S, lane, 0, detJ, g);
+        }
+        __syncthreads();
+        if (warp == 0) form_entries<DIM, 0>(S, lane, h, e, ne, A.Ke, live);
+        else if (warp == 1) form_entries<DIM, 1>(S, lane, h, e, ne, A.Ke, live);
+        else if (warp == 2) form_entries<DIM, 2>(S, lane, h, e, ne, A.Ke, live);
+        else form_entries<DIM, 3>(S, lane, h, e, ne, A.Ke, live);
+    }
+    // G_e (integral of -dN_a/dx_d over the element, exact for the 2^dim Gauss rule) and f_e (-g detJ sum_p w
+    // rho N_a on the vertical component), nodes dealt to the warps
+    const double fs = -A.gravity * detJ * (DIM == 3 ? 0.125 : 0.25);
+    for (int a = warp; a < NEN; a += 4) {
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < NEN; ++k) {
+            // sign of monomial k's term: the product of the node's signs along the monomial's axes
+            const double t = S.mom[NM + k][lane];
+            v += (__popc(k & ~a) & 1) ? -t : t;
+        }
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            double area = 1.0;
+#pragma unroll
+            for (int q = 0; q < DIM; ++q)
+                if (q != d) area *= h[q];
+            const double G = area * (DIM == 3 ? 0.25 : 0.5);
+            if (live) {
+                A.Ge[(int64_t)(a * DIM + d) * ne + e] = ((a >> d) & 1) ? -G : G;
+                A.fe[(int64_t)(a * DIM + d) * ne + e] = d == A.vert_axis ? fs * v : 0.0;
+            }
+        }
+    }
+    if (!(DIM == 3 && A.mom)) {
+        __syncthreads();
+        if (warp == 0 && live) A.Se[e] = (S.s[0][lane] + S.s[1][lane]) + (S.s[2][lane] + S.s[3][lane]);
     }
 }
 
@@ -918,7 +1007,10 @@ __global__ void __launch_bounds__(128) k_assemble_jacobian2d(AssemblyArgs A, dou
         const double peta = A.seta_in ? A.seta_in[s] : 0.0;
         const uint32_t pidx = A.perm[s];
         double derivs[9];
-        const double eta = run_rheology<2>(m, N, Tn, hasT, xg, A.max[1], peta, L, pressure, A.previous_solution,
+        double T = 0.0;
+#pragma unroll
+        for (int a = 0; a < NEN; ++a) T += N[a] * Tn[a];
+        const double eta = run_rheology<2>(m, A.info[mi], T, xg, A.max[1], peta, L, pressure, A.previous_solution,
                                            A.pfw ? A.pfw[pidx] : 0.0, nullptr, derivs, true);
         const double intFac = (A.sw ? A.sw[s] : w) * detJ;
         const double DuDx = L[0][0], DuDy = L[0][1], DvDx = L[1][0], DvDy = L[1][1];
@@ -1176,7 +1268,9 @@ void assemble(Context& c) {
     A.seta_in = c.has_peta ? c.seta_in.p : nullptr;
     A.srho_in = c.has_prho ? c.srho_in.p : nullptr;
     A.mats = c.mats.p;
+    A.info = c.mat_info.p;
     A.nmat = c.nmat;
+    axis_tables(c, A.tab);
     A.temperature = c.has_temperature ? c.temperature.p : nullptr;
     A.u = c.has_solution ? c.u_sol.p : nullptr;
     A.p = c.has_solution ? c.p_sol.p : nullptr;
@@ -1209,13 +1303,13 @@ void assemble(Context& c) {
         // (the tensor-core form writes the 27 moments instead of K_e and S_e, and its contraction
         // kernel reads them back: 2 x 216 B more per element)
         double per_el = 4.0 + packed_size(nd) * 8.0 + 2.0 * nd * 8.0 + 8.0 + (tcpath ? 2.0 * 27 * 8.0 : 0.0);
-        double flops_point = dim == 3 ? 120.0 : 50.0, flops_el = dim == 3 ? 3600.0 : 300.0;
+        double flops_point = dim == 3 ? 85.0 : 36.0, flops_el = dim == 3 ? 900.0 : 200.0;
         note_work(c, UWGPU_KERNEL_ASSEMBLY, per_point * c.np + per_el * ne, flops_point * c.np + flops_el * ne);
         LaunchScope ls(c, UWGPU_KERNEL_ASSEMBLY);
         if (dim == 3)
-            k_assemble<3><<<blocks_for(ne, 128), 128, 0, c.stream>>>(A);
+            k_assemble<3><<<blocks_for(ne, kAsEl), 128, 0, c.stream>>>(A);
         else
-            k_assemble<2><<<blocks_for(ne, 128), 128, 0, c.stream>>>(A);
+            k_assemble<2><<<blocks_for(ne, kAsEl), 128, 0, c.stream>>>(A);
     }
     check_launch("k_assemble");
     if (tcpath) {
@@ -1242,8 +1336,9 @@ void assemble(Context& c) {
     }
     check_launch("k_contract_tc");
     uint32_t flags = 0;
-    UWG_CUDA(cudaMemcpyAsync(&flags, c.err_count.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
+    UWG_CUDA(cudaMemcpyAsync(c.host_scalars, c.err_count.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
     UWG_CUDA(cudaStreamSynchronize(c.stream));
+    std::memcpy(&flags, c.host_scalars, sizeof(flags));
     c.assembled = true;
     c.operator_built = false;
     if (flags & 4u) throw Error(UWGPU_ERR_CUDA, "tensor-core contraction: an MMA did not complete in time");

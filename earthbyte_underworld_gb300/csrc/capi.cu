@@ -179,6 +179,7 @@ int uwgpu_materials_set(uwgpu_ctx* ctx, int32_t n, const uwgpu_material* mats) {
             }
         }
         upload(c.mats, mats, (size_t)n, c.stream);
+        uwg::material_info(c, n);
         UWG_CUDA(cudaStreamSynchronize(c.stream));
         c.nmat = n;
     });

@@ -147,6 +147,14 @@ struct Level {
     bool has32 = false;
 };
 
+// Per-material constants of the rheology (assembly.cu): Drucker-Prager's friction and cohesion terms per law
+// in 2D and 3D, and whether a law reads the velocity gradient.
+struct MaterialInfo {
+    double dp[4][2][2];
+    int needs_gradient;
+    int pad;
+};
+
 struct ProfileFamily {
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> events;
     size_t used = 0;
@@ -173,6 +181,7 @@ struct Context {
 
     // materials and fields
     DArray<uwgpu_material> mats;
+    DArray<MaterialInfo> mat_info;
     int nmat = 0;
     DArray<double> temperature;
     bool has_temperature = false;
@@ -380,6 +389,7 @@ void element_matrices_to_host(Context& c, int64_t first, int64_t count, const do
 void axis_tables(Context& c, const double* tab[3]);   // per axis x0[nel], h[nel], 1/h[nel] (binning.cu)
 void bin_and_map(Context& c);
 void assemble(Context& c);
+void material_info(Context& c, int n);   // from c.mats
 void strain_weakening_advance(Context& c, double dt);
 int64_t population_control(Context& c, const uwgpu_pcdvc_opts& o);
 void build_operator(Context& c, int levels, bool need32);

@@ -172,6 +172,73 @@ def _ptr(a):
     return None if a is None else a.ctypes.data
 
 
+class _HostBuffers:
+    """Memory of large result arrays, reused once the caller has dropped them.
+
+    A fresh array's pages are faulted in while the device copy writes them, at about 20 GB/s against 190 GB/s
+    into pages that are present, so a call that returns 150 MB took longer to fault than to compute.  At most
+    LIMIT bytes are held; release() gives them back.  Safe from any thread and from garbage collection inside
+    a call (the lock is re-entrant and no list is iterated while it changes)."""
+
+    LIMIT = 1 << 30
+    SMALLEST = 1 << 20
+
+    class _Block:
+        """Owner of one result's memory; numpy keeps it alive as the array's base."""
+
+        def __init__(self, pool, raw, shape, dtype):
+            self.pool, self.raw = pool, raw
+            self.__array_interface__ = dict(version=3, shape=shape, typestr=np.dtype(dtype).str,
+                                            data=(raw.ctypes.data, False))
+
+        def __del__(self):
+            try:
+                self.pool._give_back(self.raw)
+            except Exception:   # interpreter shutdown: the memory goes with the process
+                pass
+
+    def __init__(self):
+        self._lock = threading.RLock()
+        self._free = []
+        self._held = 0
+
+    def array(self, shape, dtype):
+        """an uninitialised C-ordered array"""
+        shape = (shape,) if np.isscalar(shape) else tuple(shape)
+        need = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
+        if need < self.SMALLEST:
+            return np.empty(shape, dtype)
+        raw = None
+        with self._lock:
+            fits = [k for k in range(len(self._free)) if need <= self._free[k].nbytes <= 2 * need]
+            if fits:
+                raw = self._free.pop(min(fits, key=lambda k: self._free[k].nbytes))
+                self._held -= raw.nbytes
+        if raw is None:
+            raw = np.empty(need, np.uint8)
+        return np.asarray(self._Block(self, raw, shape, dtype))
+
+    def _give_back(self, raw):
+        with self._lock:
+            while self._free and self._held + raw.nbytes > self.LIMIT:
+                self._held -= self._free.pop(0).nbytes
+            if self._held + raw.nbytes <= self.LIMIT:
+                self._free.append(raw)
+                self._held += raw.nbytes
+
+    def release(self):
+        with self._lock:
+            self._free, self._held = [], 0
+
+
+host_buffers = _HostBuffers()
+
+
+def _result(shape, dtype=np.float64):
+    """an array that a library call is about to fill entirely"""
+    return host_buffers.array(shape, dtype)
+
+
 def make_material(laws, density=0.0, alpha=0.0, ref_temp=0.0) -> Material:
     """laws: ordered list of (law_id, [params]) as in a RheologyMaterial's Rheology list."""
     if not 1 <= len(laws) <= 4:
@@ -285,7 +352,8 @@ class Context:
     def particles(self):
         """current coordinates (x, y, z) of the material points"""
         n = self.npoints
-        x, y, z = (np.zeros(n) for _ in range(3))
+        x, y = _result(n), _result(n)
+        z = _result(n) if self.dim == 3 else np.zeros(n)
         self._check(self._L.uwgpu_particles_download(self._h, _ptr(x), _ptr(y), _ptr(z) if self.dim == 3 else None))
         return x, y, z
 
@@ -293,9 +361,9 @@ class Context:
         if not want:
             self._check(self._L.uwgpu_bin_and_map(self._h, None, None, None))
             return None
-        perm = np.zeros(self.npoints, np.uint32)
-        offsets = np.zeros(self.nelements + 1, np.uint32)
-        xi = np.zeros((self.npoints, 3))
+        perm = _result(self.npoints, np.uint32)
+        offsets = _result(self.nelements + 1, np.uint32)
+        xi = _result((self.npoints, 3))
         self._check(self._L.uwgpu_bin_and_map(self._h, _ptr(perm), _ptr(offsets), _ptr(xi)))
         return perm, offsets, xi
 
@@ -309,8 +377,8 @@ class Context:
 
     def strain_weakening(self):
         """(history, time derivative from the last assembly), per point."""
-        pfw = np.zeros(self.npoints)
-        inc = np.zeros(self.npoints)
+        pfw = _result(self.npoints)
+        inc = _result(self.npoints)
         self._check(self._L.uwgpu_strain_weakening_get(self._h, _ptr(pfw), _ptr(inc)))
         return pfw, inc
 
@@ -326,8 +394,8 @@ class Context:
 
     def cell_tables(self):
         """(perm, offsets) of the current cell tables, without re-binning."""
-        perm = np.zeros(self.npoints, np.uint32)
-        offsets = np.zeros(self.nelements + 1, np.uint32)
+        perm = _result(self.npoints, np.uint32)
+        offsets = _result(self.nelements + 1, np.uint32)
         self._check(self._L.uwgpu_get_cell_tables(self._h, _ptr(perm), _ptr(offsets)))
         return perm, offsets
 
@@ -350,29 +418,31 @@ class Context:
         if count is None:
             count = self.nelements - first
         nd = (1 << self.dim) * self.dim
-        Ke = np.zeros((count, nd, nd))
-        fe = np.zeros((count, nd))
-        Ge = np.zeros((count, nd))
-        Se = np.zeros(count)
+        Ke = _result((count, nd, nd))
+        fe = _result((count, nd))
+        Ge = _result((count, nd))
+        Se = _result(count)
         self._check(self._L.uwgpu_get_element_matrices(self._h, first, count, _ptr(Ke), _ptr(fe), _ptr(Ge), _ptr(Se)))
         return Ke, fe, Ge, Se
 
     def point_viscosity(self):
-        eta = np.zeros(self.npoints)
+        eta = _result(self.npoints)
         self._check(self._L.uwgpu_get_point_viscosity(self._h, _ptr(eta)))
         return eta
 
     def operator_apply(self, x, precision=PREC_FP64):
         x = np.ascontiguousarray(x, dtype=np.float64).reshape(-1)
-        y = np.zeros_like(x)
+        y = _result(x.shape)
         self._check(self._L.uwgpu_operator_apply(self._h, precision, _ptr(x), _ptr(y)))
         return y
 
     def solve_bsscr(self, opts: SolveOpts | None = None, want=True, check=True):
         opts = opts or default_opts()
         rep = Report()
-        u = np.zeros((self.nnodes, self.dim)) if want else None
-        p = np.zeros(self.nelements) if want else None
+        # unchecked: a call that stops before it has an answer leaves zeros
+        make = _result if check else np.zeros
+        u = make((self.nnodes, self.dim)) if want else None
+        p = make(self.nelements) if want else None
         rc = self._L.uwgpu_solve_bsscr(self._h, C.byref(opts), _ptr(u), _ptr(p), C.byref(rep))
         if check:
             self._check(rc)
@@ -434,8 +504,8 @@ class Context:
     def integration_points(self):
         """(local coordinates [slot][3], weights [slot]) the last assembly integrated with."""
         n = self.npoints
-        xi = np.zeros((n, 3))
-        w = np.zeros(n)
+        xi = _result((n, 3))
+        w = _result(n)
         self._check(self._L.uwgpu_integration_points(self._h, _ptr(xi), _ptr(w)))
         return xi, w
 

@@ -8,8 +8,8 @@
 // the FP32 rate) makes every CG iteration FP64-issue bound.  The stencil is built once per solve
 // (A[q][e], entry-major, q = neighbour offset) and an iteration is then 27 FMAs per element
 // with coalesced stencil reads; the 57 MB FP64 stencil of a 64^3 mesh can stay in L2.  In FP32
-// the matrix-free chain is cheap, so the mixed form applies G^T W G matrix-free (k_cg_mf3_dir,
-// k_cg_mf2_dir below) once its FP32 stencil would no longer fit in L2.
+// the matrix-free chain is cheap, so the mixed form applies G^T W G matrix-free (k_cg_mf3_dir_tma,
+// k_cg_mf3_dir, k_cg_mf2_dir below) where that is faster than its FP32 stencil.
 // Further down: the aggregation multigrid option for the inner solves, and the test and timing
 // hooks on the inner operator.
 //
@@ -889,8 +889,7 @@ __global__ void k_mf_weights(int64_t nn, int dim, int64_t nnx, int64_t nny, int6
 
 
 
-// the launch of the matrix-free direction kernel: in 3D the deepest column chunk (up to 16
-// element planes) that still gives four blocks per SM, at least 2 planes
+// the launch of the matrix-free direction kernel
 struct MfLaunch {
     int dim;
     int ex, ey;
@@ -941,8 +940,22 @@ static MfLaunch mf_launch(const MeshDesc& m, EGrid g, const float* Wc, const flo
         L.blocks = (unsigned)txy;
         return L;
     }
-    int zc = 16;
-    while (zc > 2 && txy * ((g.ez + zc - 1) / zc) < 4 * (int64_t)sms) zc /= 2;
+    // z chunk: a block forms zc + 2 stages for zc element planes, one after the other.  Measured on the TMA
+    // kernel (us per launch, chunks of 2 to 32 planes on 24^3 to 128^3 meshes): a stage takes 0.54 us in a
+    // block alone on its SM and 0.225 us per resident block when they share it (up to four), a wave 1.2 us
+    // besides.  The chunk with the least of that is within 5% of the best one tried: 64 x 80 x 112 8.50 us
+    // (two planes) -> 6.63 (four), 96^3 10.5 -> 8.3, 128^3 17.7 -> 16.7, 64^3 4.9 and below unchanged.
+    int zc = 1;
+    double best = 1e300;
+    for (int t = 1; t <= 64 && t <= g.ez; ++t) {
+        const int64_t blocks = txy * ((g.ez + t - 1) / t), per_sm = (blocks + sms - 1) / sms;
+        const double waves = (double)((blocks + 4 * (int64_t)sms - 1) / (4 * (int64_t)sms));
+        const double cost = waves * ((t + 2) * std::max(0.54, 0.225 * (double)std::min<int64_t>(per_sm, 4)) + 1.2);
+        if (cost < best) {
+            best = cost;
+            zc = t;
+        }
+    }
     const int64_t pitch = (m.nnx + 3) / 4 * 4;
     L.a3 = Mf3{(int)g.ex, (int)g.ey, (int)g.ez, zc, pitch, m.nny, pitch * m.nny * m.nnz};
     L.blocks = (unsigned)(txy * ((g.ez + zc - 1) / zc));
@@ -1598,11 +1611,6 @@ static int gwg_cg_T(Context& c, const T* A, const float* Wmf, const T* dinv, con
         LaunchScope ls(c, UWGPU_KERNEL_VECTOR);
         dir(-1, 1);
     }
-    double* hs = c.host_scalars;
-    UWG_CUDA(cudaMemcpyAsync(hs, scal, 8 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    UWG_CUDA(cudaStreamSynchronize(c.stream));
-    const double r0 = std::sqrt(hs[7]);
-    if (!(r0 > 0.0)) return 0;
     // Twelve iterations (the rz slots cycle with period 3, pq and rr with period 2) form one CUDA
     // graph per buffer set, replayed until converged; the host checks the residual once per replay.
     const int block = 12;
@@ -1634,8 +1642,17 @@ static int gwg_cg_T(Context& c, const T* A, const float* Wmf, const T* dinv, con
     // weights of about one node per element in place of the stencil)
     const double it_bytes = (double)ne * sizeof(T) * (8 + (Wmf ? m.dim : nb) + 5 + (cc ? 3 : 0));
     const double it_flops = Wmf ? (double)ne * (m.dim == 3 ? 110.0 : 46.0) : (double)ne * (2.0 * nb + 14.0);
-    int it = 0;
-    while (it < maxit) {
+    // The next replay is queued before the last one's residual is known while that of the one before is
+    // more than kFar times the tolerance away (the residual falls by a few percent per replay), so the GPU
+    // does not wait for the host: a replay of 185 us used to be followed by 25 us of idle time.  Near the
+    // tolerance, and before anything is known, the host looks first; a replay queued in vain leaves x nearer
+    // to the solution.  The FP64 form stops exactly where the test says.
+    constexpr double kFar = sizeof(T) == 4 ? 4.0 : 1e300;
+    for (auto& ev : c.pcg_events)
+        if (!ev) UWG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    double* hs = c.host_scalars;
+    int it = 0, queued = 0, seen = 0;   // iterations and replays queued, replays whose residual has been read
+    auto queue = [&]() {
         {
             LaunchScope ls(c, UWGPU_KERNEL_SCHUR_PC);
             UWG_CUDA(cudaGraphLaunch(pg->exec, c.stream));
@@ -1643,11 +1660,29 @@ static int gwg_cg_T(Context& c, const T* A, const float* Wmf, const T* dinv, con
         note_work(c, UWGPU_KERNEL_SCHUR_PC, block * it_bytes, block * it_flops);
         c.launches += (cc ? 5 : 2) * block - 1;
         it += block;
-        UWG_CUDA(cudaMemcpyAsync(hs, scal, 8 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-        UWG_CUDA(cudaStreamSynchronize(c.stream));
-        const double rn = std::sqrt(hs[6]);   // rr of the block's last iteration (k = 11: slot 5 + 1)
+        const int slot = queued++ & 1;
+        UWG_CUDA(cudaMemcpyAsync(hs + 8 * slot, scal, 8 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+        UWG_CUDA(cudaEventRecord(c.pcg_events[slot], c.stream));
+    };
+    double ratio = 0.0;   // last known ||r|| over its tolerance
+    while (true) {
+        if (queued == seen) {
+            if (it >= maxit) break;
+            queue();
+        }
+        if (it < maxit && ratio > kFar && queued == seen + 1) queue();
+        const double* h = hs + 8 * (seen & 1);
+        UWG_CUDA(cudaEventSynchronize(c.pcg_events[seen & 1]));
+        ++seen;
+        const double r0 = std::sqrt(h[7]);
+        if (!(r0 > 0.0)) {   // nothing to solve: x = 0
+            UWG_CUDA(cudaMemsetAsync(x, 0, (size_t)ne * sizeof(T), c.stream));
+            return 0;
+        }
+        const double rn = std::sqrt(h[6]);   // rr of the block's last iteration (k = 11: slot 5 + 1)
         if (!std::isfinite(rn)) throw Error(UWGPU_ERR_NAN, "NaN in the BFBt inner solve");
         if (rn <= rtol * r0) break;
+        ratio = rn / (rtol * r0);
     }
     check_launch("gwg_cg");
     return it;

@@ -290,6 +290,7 @@ struct Context {
         DArray<double> einv, s, y, ed;
     } cc;
     std::vector<PcgGraph> pcg_graphs;
+    cudaEvent_t pcg_events[2] = {nullptr, nullptr};   // the residuals of two queued replays
 
     // learned velocity preconditioner (csrc/unet.cu), created on request
     unet::Net* net = nullptr;
@@ -298,6 +299,8 @@ struct Context {
         unet::destroy(net);
         for (auto& g : pcg_graphs)
             if (g.exec) cudaGraphExecDestroy(g.exec);
+        for (auto ev : pcg_events)
+            if (ev) cudaEventDestroy(ev);
     }
 };
 

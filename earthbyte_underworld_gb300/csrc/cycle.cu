@@ -16,6 +16,14 @@
 // the work of a block is packed into as few warps as hold it.  What a smoothing call does not change
 // (stencil, inverse diagonal, right-hand side) is fetched between arriving at a barrier and waiting on it.
 //
+// In 2D the colours of a Gauss-Seidel call, most of a cycle's phases, are not separated by barriers: every
+// value is kept beside a tag that names the step that formed it, in one word that is read and written whole,
+// and a row polls its neighbours until each carries the tag of its colour's last step.  A node cannot be
+// relaxed again before its neighbours have used the value (its next relaxation waits for theirs), so the
+// colours follow each other through the data.  Per V-cycle iteration: 65^2 237 -> 196 us, 129^2 255 -> 210,
+// 257^2 393 -> 349.  In 3D a thread polls 27 words instead of 6 and the barrier is the faster (17^3 456 us
+// against 525).
+//
 // Vectors written during the launch are read past L1 (__ldcg).  The arithmetic is that of the per-kernel
 // path (operator.cu, solver.cu) up to the order of sums.
 #include <cuda_fp16.h>
@@ -33,13 +41,61 @@ namespace {
 constexpr int kCyThreads = 256;
 constexpr int kCyKrylovBlocks = 64;     // blocks of the Gram-Schmidt part (each adds up all partial sums)
 constexpr int kCyWait = 1 << 22;        // polls of a barrier before the launch gives up
+constexpr int kCyPolls = 1 << 20;       // polls of a row's neighbours
+constexpr int kCySweeps = 256;          // most smoothing sweeps per call
 // Levels (nodes) up to which the cycle runs here, per smoother, measured per V-cycle iteration of whole
 // velocity solves (us, all levels as separate kernels / this level and below here): colour sweeps, which
-// alternate with barriers, 2D 65^2 461 / 237, 129^2 490 / 255, 257^2 547 / 393; 3D 17^3 1167 / 456, 33^3
+// alternate with barriers, 2D 65^2 461 / 196, 129^2 490 / 210, 257^2 547 / 349; 3D 17^3 1167 / 456, 33^3
 // 1408 / 781, 41^3 1986 / 1254 (81,000 nodes and more were not tried, the kernels win at 65^3: 1014
 // against 585 with Chebyshev).  Chebyshev in mixed precision: 17^3 226 / 117, 33^3 289 / 215 with the whole
 // iteration here; as levels below a 65^3 mesh 17^3 and less gain (585 / 577), 33^3 does not (590).
 constexpr int64_t kCyNodesColour = 80000, kCyNodesCheb = 6000, kCyNodesWhole = 40000;
+
+// A value and the tag of the step that formed it, in one naturally aligned word of 16 or 8 bytes
+template <typename T>
+struct alignas(2 * sizeof(T)) Tagged {
+    T v;
+    uint32_t tag;
+};
+__device__ __forceinline__ Tagged<double> load_tagged(const Tagged<double>* p) {
+    uint64_t a, b;
+    asm volatile("{ .reg .b128 q; ld.relaxed.gpu.global.b128 q, [%2]; mov.b128 {%0, %1}, q; }" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+    return Tagged<double>{__longlong_as_double((long long)a), (uint32_t)b};
+}
+__device__ __forceinline__ void store_tagged(Tagged<double>* p, double v, uint32_t tag) {
+    asm volatile("{ .reg .b128 q; mov.b128 q, {%1, %2}; st.relaxed.gpu.global.b128 [%0], q; }" ::"l"(p),
+                 "l"(__double_as_longlong(v)), "l"((uint64_t)tag)
+                 : "memory");
+}
+__device__ __forceinline__ Tagged<float> load_tagged(const Tagged<float>* p) {
+    uint64_t a;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
+    return Tagged<float>{__uint_as_float((uint32_t)a), (uint32_t)(a >> 32)};
+}
+__device__ __forceinline__ void store_tagged(Tagged<float>* p, float v, uint32_t tag) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((uint64_t)__float_as_uint(v) | (uint64_t)tag << 32) : "memory");
+}
+
+// Last step before `step` of the triangle wave of colours (gs_step_colour) that relaxed colour c; -1: none
+template <int DIM>
+__host__ __device__ constexpr int last_step(int step, int c) {
+    constexpr int P = (1 << DIM) - 1;
+    const int q = step % (2 * P), base = step - q;
+    const int down = c == 0 ? 2 * P : 2 * P - c;   // the colour's descending place in a period (0: the next period)
+    if (down < q) return base + down;
+    if (c < q) return base + c;
+    return base == 0 ? -1 : base - 2 * P + (c == 0 ? 0 : 2 * P - c);
+}
+constexpr bool last_step_ok() {
+    int last[4] = {-1, -1, -1, -1};
+    for (int step = 0; step < gs_steps<2>(3); ++step) {
+        for (int c = 0; c < 4; ++c)
+            if (last_step<2>(step, c) != last[c]) return false;
+        last[gs_step_colour<2>(step)] = step;
+    }
+    return true;
+}
+static_assert(last_step_ok(), "last_step and gs_step_colour disagree");
 
 template <typename T>
 struct CyLevel {
@@ -49,6 +105,7 @@ struct CyLevel {
     const float* S16;
     const T* Dinv;
     T *b, *x, *r, *t;      // right-hand side, iterate, residual or Chebyshev direction, alternate iterate
+    Tagged<T>* xt;         // 2D: the iterate with the tags of a Gauss-Seidel call
     const uint8_t* fixed;
     T c1[kCyMaxDegree], c2[kCyMaxDegree];   // Chebyshev recurrence (k_cheb_step)
 };
@@ -61,6 +118,7 @@ struct CyArgs {
     int64_t ncoarse;
     uint32_t* bar;         // [0] this launch's barrier count, [1] the next launch's (cleared here), [2] error
     int which;             // which of the two counts this launch uses
+    uint32_t tag;          // first tag of this launch (2D)
     int64_t n;             // unknowns of the finest level
     // Krylov part (V null: the cycle alone): vectors V_j of n entries, j <= k
     const T* V;
@@ -129,6 +187,46 @@ struct RowThird {
 #pragma unroll
                 for (int cc = 0; cc < DIM; ++cc) a[t * DIM + cc] = __ldg(p + (t * DIM * DIM + cc) * nn);
         }
+    }
+    // 2D: the product with the tagged iterate; polls until every neighbour carries its colour's last tag before
+    // `step` (tag0 for the initial values; zero: those are zero and nothing is read); false when it gave up
+    __device__ __forceinline__ bool dot_tagged(const CyLevel<T>& L, int n, int s, int col, int step, uint32_t tag0, bool zero,
+                                               bool poll, T& out) const {
+        static_assert(DIM == 2, "the tagged iterate is the 2D form");
+        const Grid& g = L.g;
+        const int nn = (int)g.nn, nx = (int)g.nx;
+        int64_t i, j, k;
+        node_ijk<DIM>(g, n, i, j, k);
+        const bool in = s == 0 ? j > 0 : s == 1 || j + 1 < g.ny;   // the third (row j + s - 1) lies in the mesh
+        const int row = n + (s - 1) * nx;
+        uint32_t want[2];   // tag to wait for, of the neighbours in this and in the next columns; 0: nothing to read
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int last = last_step<DIM>(step, (s == 1 ? col : col ^ 2) ^ q);
+            want[q] = last < 0 ? (zero ? 0u : tag0) : tag0 + 1u + (uint32_t)last;
+        }
+        const bool live[3] = {in && i > 0 && want[1], in && want[0], in && i + 1 < g.nx && want[1]};
+        T xv[NQ * DIM];
+        bool ready;
+        int polls = 0;
+        do {
+            ready = true;
+#pragma unroll
+            for (int t = 0; t < NQ; ++t)
+#pragma unroll
+                for (int cc = 0; cc < DIM; ++cc) {
+                    xv[t * DIM + cc] = (T)0;
+                    if (live[t]) {
+                        const Tagged<T> e = load_tagged(L.xt + cc * nn + row + t - 1);
+                        xv[t * DIM + cc] = e.v;
+                        ready = ready && e.tag == want[(t + 1) & 1];
+                    }
+                }
+        } while (!ready && poll && ++polls < kCyPolls);
+        out = (T)0;
+#pragma unroll
+        for (int t = 0; t < NQ * DIM; ++t) out = fma(a[t], xv[t], out);
+        return ready;
     }
     __device__ __forceinline__ T dot(const CyLevel<T>& L, int n, int s, const T* x) const {
         const Grid& g = L.g;
@@ -255,17 +353,24 @@ __device__ __forceinline__ void node_phase(const CyLevel<T>& L, const T* x, T* y
 
 template <int DIM, typename T, bool HALF>
 __global__ void __launch_bounds__(kCyThreads, 1) k_cycle(const __grid_constant__ CyArgs<T> a) {
-    __shared__ T sres[kCyThreads];
+    __shared__ T sres[2 * kCyThreads];
     __shared__ double s_h[kCyPass];
+    __shared__ int s_dead;   // a poll of this block has run out: no more polling
     const int tid = threadIdx.x, gt = (int)blockIdx.x * kCyThreads + tid, gn = (int)gridDim.x * kCyThreads;
     constexpr int W = 3 * DIM, ROUND = kCyThreads / W;
     GridBarrier bar{a.bar + a.which, a.bar + 2};
     if (gt == 0) a.bar[a.which ^ 1] = 0u;   // the next launch's count
+    if (tid == 0) s_dead = 0;
+    __syncthreads();
 
     // symmetric colour Gauss-Seidel (gs_steps, gs_step_colour).  A barrier may be pending on entry, and one
-    // is on exit: whoever needs the values waits.  b and the stencil do not change here.
-    auto smooth_gs = [&](const CyLevel<T>& L, int sweeps) {
+    // is on exit: whoever needs the values waits.  b and the stencil do not change here.  2D: on the tagged
+    // iterate, from zero or from the values stored with tag `tag`; the block's partial sums alternate between
+    // two buffers, so one block barrier per round orders them.
+    uint32_t tag = a.tag;
+    auto smooth_gs = [&](const CyLevel<T>& L, int sweeps, bool zero) {
         const int steps = gs_steps<DIM>(sweeps), nn = (int)L.g.nn;
+        int buf = 0;
         for (int st = 0; st < steps; ++st) {
             const int col = gs_step_colour<DIM>(st), px = col & 1, py = (col >> 1) & 1, pz = (col >> 2) & 1;
             const int cx = (int)(L.g.nx - px + 1) / 2, cy = (int)(L.g.ny - py + 1) / 2;
@@ -292,28 +397,46 @@ __global__ void __launch_bounds__(kCyThreads, 1) k_cycle(const __grid_constant__
                         }
                     }
                 }
-                if (base == 0) bar.wait();
-                else __syncthreads();   // the previous round's sums have been read
-                if (act) {
-                    if (combo < DIM) v = __ldcg(L.x + combo * nn + n);
-                    sres[tid] = row.dot(L, n, combo % 3, L.x);
+                T* sb = sres + buf * kCyThreads;
+                if constexpr (DIM == 2) {
+                    buf ^= 1;
+                    bar.wait();   // (pending in the first round of the call only)
+                    if (act) {
+                        // the node's own value: this thread stored it in an earlier step, or another before the barrier
+                        if (combo < DIM && !(zero && last_step<DIM>(st, col) < 0)) v = load_tagged(L.xt + combo * nn + n).v;
+                        T part;
+                        if (!row.dot_tagged(L, n, combo % 3, col, st, tag, zero, !s_dead, part)) {
+                            if (!s_dead) atomicOr(a.bar + 2, 1u);
+                            s_dead = 1;
+                        }
+                        sb[tid] = part;
+                    }
+                } else {
+                    if (base == 0) bar.wait();
+                    else __syncthreads();   // the previous round's sums have been read
+                    if (act) {
+                        if (combo < DIM) v = __ldcg(L.x + combo * nn + n);
+                        sb[tid] = row.dot(L, n, combo % 3, L.x);
+                    }
                 }
                 __syncthreads();
                 if (act && combo < DIM) {
 #pragma unroll
                     for (int cc = 0; cc < DIM; ++cc) {
-                        const T* p = sres + cc * 3 * cnt + loc;
+                        const T* p = sb + cc * 3 * cnt + loc;
                         v = fma(dv[cc], bv[cc] - ((p[0] + p[cnt]) + p[2 * cnt]), v);
                     }
+                    if (DIM == 2) store_tagged(L.xt + combo * nn + n, v, tag + 1u + (uint32_t)st);
                     L.x[combo * nn + n] = v;
                 }
             }
-            bar.arrive();
+            if (DIM == 3 || st + 1 == steps) bar.arrive();
         }
+        tag += (uint32_t)steps + 2u;
     };
     auto smooth = [&](const CyLevel<T>& L, int sweeps, bool zero) {
         if (!a.cheb) {
-            smooth_gs(L, sweeps);
+            smooth_gs(L, sweeps, zero);
             return;
         }
         const T* cur = zero ? nullptr : L.x;
@@ -399,7 +522,9 @@ __global__ void __launch_bounds__(kCyThreads, 1) k_cycle(const __grid_constant__
                 const bool live = in && !__ldg(C.fixed + N * DIM + d);
                 acc = fma(w, live ? v : (T)0, acc);
             }
-            if (!__ldg(F.fixed + n * DIM + d)) F.x[it] = __ldcg(F.x + it) + acc;
+            const T old = __ldcg(F.x + it), v = __ldg(F.fixed + n * DIM + d) ? old : old + acc;
+            F.x[it] = v;
+            if (DIM == 2 && !a.cheb) store_tagged(F.xt + it, v, tag);   // the smoother's initial values
         }
         bar.arrive();
         smooth(F, a.up, false);
@@ -500,6 +625,29 @@ void launch(Context& c, CyArgs<T>& a) {
     a.bar = c.cycle_bar.p;
     a.which = c.cycle_which;
     a.part = c.cycle_part.p;
+    if (DIM == 2 && !a.cheb) {
+        // tagged iterates of the levels, and tags that no earlier launch has used; a word keeps the place and
+        // type it had, or starts again from tag 0
+        size_t bytes = 0;
+        for (int l = 0; l + 1 < a.nlev; ++l) bytes += (size_t)a.L[l].g.nn * DIM * sizeof(Tagged<T>);
+        const uint64_t tags = (uint64_t)a.nlev * (gs_steps<DIM>(a.down) + gs_steps<DIM>(a.up) + 4);
+        const uint64_t layout[3] = {(uint64_t)a.L[0].g.nx, (uint64_t)a.L[0].g.ny, (uint64_t)a.nlev * 16 + sizeof(T)};
+        const bool fresh = c.cycle_tagged.n * sizeof(uint64_t) < bytes ||
+                           !std::equal(layout, layout + 3, c.cycle_layout);
+        c.cycle_tagged.ensure((bytes + 15) / 16 * 2);
+        if (fresh || c.cycle_tag + tags > 0xffffffffull) {
+            UWG_CUDA(cudaMemsetAsync(c.cycle_tagged.p, 0, c.cycle_tagged.n * sizeof(uint64_t), c.stream));
+            c.cycle_tag = 1;
+            std::copy(layout, layout + 3, c.cycle_layout);
+        }
+        unsigned char* at = reinterpret_cast<unsigned char*>(c.cycle_tagged.p);
+        for (int l = 0; l + 1 < a.nlev; ++l) {
+            a.L[l].xt = reinterpret_cast<Tagged<T>*>(at);
+            at += (size_t)a.L[l].g.nn * DIM * sizeof(Tagged<T>);
+        }
+        a.tag = (uint32_t)c.cycle_tag;
+        c.cycle_tag += tags;
+    }
     void* args[] = {(void*)&a};
     UWG_CUDA(cudaLaunchCooperativeKernel((const void*)k_cycle<DIM, T, HALF>, dim3((unsigned)sms), dim3(kCyThreads), args, 0,
                                          c.stream));
@@ -574,7 +722,7 @@ void run(Context& c, CyArgs<T>& a) {
 
 int cycle_first_level(const Context& c, const CycleOpts& o) {
     const int nlev = c.nlevels;
-    if (nlev < 2 || o.cycle != 1 || o.down < 0 || o.up < 0) return nlev;
+    if (nlev < 2 || o.cycle != 1 || o.down < 0 || o.up < 0 || o.down > kCySweeps || o.up > kCySweeps) return nlev;
     if (o.cheb && (o.down > kCyMaxDegree || o.up > kCyMaxDegree || o.down < 1)) return nlev;
     if (c.levels[nlev - 1].ncoarse > 4000) return nlev;
     const int64_t limit = !o.cheb ? kCyNodesColour : c.levels[0].mesh.nn <= kCyNodesWhole ? kCyNodesWhole : kCyNodesCheb;

@@ -250,6 +250,9 @@ struct Context {
     DArray<uint32_t> cycle_bar;
     DArray<double> cycle_part;
     int cycle_which = 0;
+    DArray<uint64_t> cycle_tagged;   // 2D iterates with the tags of the steps that formed them
+    uint64_t cycle_tag = 1;          // next unused tag
+    uint64_t cycle_layout[3] = {0, 0, 0};
     DArray<double> io;        // staging of transfers to and from the host (hostio.cu)
     DArray<double> io_x, io_y;   // vectors of uwgpu_operator_apply
     double* host_scalars = nullptr;   // pinned

@@ -266,10 +266,14 @@ constexpr int kEpt = 2;
 // kernel then updates x); r -= alpha q; z = dinv r; rz_{k+1} += r.z; and, when want_rr (the host's
 // convergence check follows), rr_k += r.r.  Clears the slots of rz_{k+2} and pq_{k+1}.
 // k_cg_update: 512 threads x 4 elements per block, so that few blocks (1,024 at 128^3) add their
-// partial sums to the same two scalars (same-address atomics serialise in L2)
+// partial sums to the same two scalars (same-address atomics serialise in L2).  On small grids that leaves
+// most SMs idle while each thread works through its elements and thread 0 through the warps' sums, in FP64
+// at 64 cycles an instruction: up to kCgSmall elements a block is 128 threads x 1 element, and the stencil
+// kernel 64 threads.
 constexpr int kUpdThreads = 512, kUpdEpt = 4;
+constexpr int64_t kCgSmall = 65536;
 
-template <typename T>
+template <typename T, int EPT>
 __global__ void __launch_bounds__(kUpdThreads) k_cg_update(int64_t ne, const T* __restrict__ p, const T* __restrict__ q,
                             const T* __restrict__ dinv, T* __restrict__ x, T* __restrict__ r, T* __restrict__ z,
                             double* __restrict__ scal, int k, int want_rr, int with_x) {
@@ -277,10 +281,10 @@ __global__ void __launch_bounds__(kUpdThreads) k_cg_update(int64_t ne, const T* 
     __shared__ T s_alpha;
     pdl_wait();
     // the vectors first: their loads are in flight while thread 0 fetches the scalars for alpha
-    const int64_t base = (int64_t)blockIdx.x * blockDim.x * kUpdEpt + threadIdx.x;
-    T pv[kUpdEpt], qv[kUpdEpt], xv[kUpdEpt], rv[kUpdEpt], dv[kUpdEpt];
+    const int64_t base = (int64_t)blockIdx.x * blockDim.x * EPT + threadIdx.x;
+    T pv[EPT], qv[EPT], xv[EPT], rv[EPT], dv[EPT];
 #pragma unroll
-    for (int m = 0; m < kUpdEpt; ++m) {
+    for (int m = 0; m < EPT; ++m) {
         const int64_t e = base + (int64_t)m * blockDim.x;
         const bool in = e < ne;
         pv[m] = in && with_x ? p[e] : (T)0;
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(kUpdThreads) k_cg_update(int64_t ne, const T* 
     const T alpha = block_ratio<T>(rz_slot(scal, k), pq_slot(scal, k), &s_alpha);
     T rz = (T)0, rr = (T)0;
 #pragma unroll
-    for (int m = 0; m < kUpdEpt; ++m) {
+    for (int m = 0; m < EPT; ++m) {
         const int64_t e = base + (int64_t)m * blockDim.x;
         if (e < ne) {
             if (with_x) x[e] = fma(alpha, pv[m], xv[m]);
@@ -1595,8 +1599,9 @@ static int gwg_cg_T(Context& c, const T* A, const float* Wmf, const T* dinv, con
                 return;
             }
         }
-        if (m.dim == 3) launch_pdl(k_cg_spmv_dir<3, T>, eb, 256, c.stream, g, A, z, p, q, scal, k, first);
-        else launch_pdl(k_cg_spmv_dir<2, T>, eb, 256, c.stream, g, A, z, p, q, scal, k, first);
+        const unsigned nt = ne <= kCgSmall ? 64u : 256u;
+        if (m.dim == 3) launch_pdl(k_cg_spmv_dir<3, T>, blocks_for(ne, (int)nt), nt, c.stream, g, A, z, p, q, scal, k, first);
+        else launch_pdl(k_cg_spmv_dir<2, T>, blocks_for(ne, (int)nt), nt, c.stream, g, A, z, p, q, scal, k, first);
     };
     // the plane-checkerboard coarse correction, when the solver built it for this operator
     const bool cc = c.cc.on && m.dim == 3 && c.cc.ex == g.ex && c.cc.ey == g.ey && c.cc.ez == g.ez;
@@ -1615,8 +1620,12 @@ static int gwg_cg_T(Context& c, const T* A, const float* Wmf, const T* dinv, con
     // graph per buffer set, replayed until converged; the host checks the residual once per replay.
     const int block = 12;
     auto issue = [&](int k) {
-        launch_pdl(k_cg_update<T>, blocks_for(ne, kUpdThreads * kUpdEpt), (unsigned)kUpdThreads, c.stream, ne, p, q, dinv,
-                   x, r, z, scal, k, (int)(k == block - 1), (int)!fused_x);
+        if (ne <= kCgSmall)
+            launch_pdl(k_cg_update<T, 1>, blocks_for(ne, 128), 128u, c.stream, ne, p, q, dinv, x, r, z, scal, k,
+                       (int)(k == block - 1), (int)!fused_x);
+        else
+            launch_pdl(k_cg_update<T, kUpdEpt>, blocks_for(ne, kUpdThreads * kUpdEpt), (unsigned)kUpdThreads, c.stream, ne, p,
+                       q, dinv, x, r, z, scal, k, (int)(k == block - 1), (int)!fused_x);
         if (cc) cc_apply<T>(c, r, z, scal, k);
         dir(k, 0);
     };

@@ -64,6 +64,18 @@ __device__ __forceinline__ uint64_t mn_major_desc(uint32_t base, int s, int rdim
     return smem_desc(base + (uint32_t)s * 2u * (uint32_t)rdim * 16u, (uint32_t)rdim * 16u, 128u);
 }
 
+// True in one thread of a converged warp.  A branch on a warp-uniform condition and this lets the compiler
+// keep the descriptors of the MMAs inside it in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)::"memory");
+    return ok != 0;
+}
+
 // ---- TMEM allocation (one whole warp executes these) ----
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)),

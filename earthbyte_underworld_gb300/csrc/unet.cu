@@ -64,9 +64,7 @@ __device__ __forceinline__ void store8(float* p, const float v[8]) {
 // carries about 16 significant bits (the split of Henry, Tang and Heinecke, "Leveraging the
 // bfloat16 artificial intelligence datatype for higher-precision computations", ARITH 2019);
 // both parts are multiplied on the tensor core and accumulated in FP32.
-__device__ __forceinline__ void split8(const float* p, uint4& hi, uint4& lo) {
-    float v[8];
-    load8(p, v);
+__device__ __forceinline__ void split8(const float v[8], uint4& hi, uint4& lo) {
     __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&hi);
     __nv_bfloat162* l = reinterpret_cast<__nv_bfloat162*>(&lo);
 #pragma unroll
@@ -78,143 +76,268 @@ __device__ __forceinline__ void split8(const float* p, uint4& hi, uint4& lo) {
     }
 }
 
-constexpr int kTcSmemBudget = 200 * 1024;   // dynamic shared memory a tensor-core conv kernel may use
+// Both convolution kernels work on tiles of 8 voxels in x by some rows in y of one z plane and
+// stage, per chunk of 8 channels, the tile with its halo as [y][x] rows of 16 bytes.  Eight
+// consecutive x of a row are then one 128-byte core matrix and consecutive y are a fixed stride
+// apart, so the operand of a tap (dx, dy) is the staged tile at a shifted start address: a tile is
+// read 4.2 times (three z planes of 10 x 18 for 8 x 16) instead of once per tap.  Staging is by
+// 16-byte cp.async with zero fill outside the grid, into a ring of stages.
+constexpr int kTx = 8, kTy = 16, kHx = kTx + 2;
+constexpr int kConvThreads = 256;
+constexpr int kConvStages = 4;                   // most stages of a ring
+constexpr size_t kSmemTwo = 108 * 1024;          // dynamic shared memory with which two CTAs share an SM
+constexpr size_t kSmemOne = 216 * 1024;
+constexpr size_t kSmemWidth = 227 * 1024 - 64;    // see conv_launch_tc
 
-// Shared-memory plan of k_conv3_tc: B (the weights) for all 27 taps when they fit, else two tap
-// buffers; A double-buffered per tap, with a second (lo) part for FP32 inputs.
-struct ConvTcPlan {
-    int Kp, Np;
-    int resident;
-    size_t bytesB, bytesA, smem;
+// rows of a chunk, padded so that the 16-byte stores of eight consecutive threads (channels
+// fastest, `kc8` chunks) fall in different banks
+__host__ __device__ inline int chunk_rows(int rows, int kc8) {
+    const int w = kc8 >= 8 ? 1 : 8 / kc8;
+    return rows + ((w - rows) % 8 + 8) % 8;
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// at most `ahead` (0, 1 or 2) of this thread's groups still in flight
+__device__ __forceinline__ void cp_wait(int ahead) {
+    if (ahead == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else if (ahead == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 2;" ::: "memory");
+}
+// stages of a ring that loads `ahead` stages before the one being multiplied: with one more stage
+// than that, the load waits for the MMAs just issued; with two more, for those before
+__host__ __device__ inline int ring_ahead(int stages) { return stages >= 4 ? 2 : stages >= 2 ? 1 : 0; }
+
+// completion of the stages of a ring, in order; every wait is bounded
+struct RingWait {
+    uint64_t* bar;
+    int stages;
+    int done = 0, slot = 0;   // stages known complete, slot of the next
+    uint32_t parity = 0;
+    __device__ __forceinline__ bool upto(int i, uint32_t limit = 1u << 22) {
+        bool ok = true;
+        for (; done <= i; ++done) {
+            ok = tc::mbar_wait(&bar[slot], parity, limit) && ok;
+            if (++slot == stages) {
+                slot = 0;
+                parity ^= 1u;
+            }
+        }
+        return ok;
+    }
 };
-__host__ __device__ inline ConvTcPlan conv_tc_plan(int K, int N, bool split) {
-    ConvTcPlan p;
-    p.Kp = (K + 15) / 16 * 16;
-    p.Np = (N + 15) / 16 * 16;
-    p.bytesB = (size_t)p.Np * p.Kp * 2;
-    p.bytesA = (size_t)128 * p.Kp * 2;
-    const size_t a_total = 2 * (split ? 2 : 1) * p.bytesA;
-    p.resident = 27 * p.bytesB + a_total <= (size_t)kTcSmemBudget ? 1 : 0;
-    p.smem = (p.resident ? 27 : 2) * p.bytesB + a_total;
-    return p;
+
+// Plan of k_conv3_tc.  A stage is the input of nine taps (one z plane of the halo) or three (one
+// y shift of it, where nine do not fit) and, unless the weights of all taps stay resident, these
+// taps' weights.
+struct ConvPlan {
+    int kc8;             // chunks of 8 input channels (even: K is padded to 16)
+    int Nc, nchunks;     // output channels per CTA, and CTAs (grid.y) that share the channels
+    int taps;            // 9 or 3
+    int stages, resident;
+    uint32_t chunkA, chunkB, partA, tapB, stage;   // bytes
+    size_t smem;
+};
+inline bool conv_plan_try(ConvPlan& p, int K, int parts, int taps, bool resident, int least, int most, size_t budget) {
+    p.kc8 = (K + 15) / 16 * 2;
+    p.taps = taps;
+    p.resident = resident;
+    p.chunkA = (uint32_t)chunk_rows((taps == 9 ? kTy + 2 : kTy) * kHx, p.kc8) * 16u;
+    p.chunkB = (uint32_t)chunk_rows(p.Nc, p.kc8) * 16u;
+    p.partA = p.kc8 * p.chunkA;
+    p.tapB = p.kc8 * p.chunkB;
+    p.stage = (uint32_t)parts * p.partA + (resident ? 0u : (uint32_t)taps * p.tapB);
+    const size_t fixed = resident ? (size_t)27 * p.tapB : 0;
+    if (fixed >= budget) return false;
+    const int64_t n = (int64_t)((budget - fixed) / p.stage);
+    p.stages = (int)(n < most ? n : most);
+    p.smem = fixed + (size_t)p.stages * p.stage;
+    return p.stages >= least;
+}
+// `tiles` voxel tiles on `sms` SMs.  The output channels are shared out (16 at least per CTA)
+// while there are fewer than two CTAs per SM: the coarse levels have 7 or 28 tiles (128 -> 128 channels on
+// 7 x 7 x 7 voxels: 153 us on three CTAs, 16 us on 56).  Weights stay resident where a CTA runs over several
+// tiles.  Nine taps per stage read the halo once; three where two stages of nine do not fit.
+inline ConvPlan conv_plan(int K, int N, int parts, int64_t tiles, int sms) {
+    const int n16 = (N + 15) / 16;
+    int want = (int)((2 * (int64_t)sms + tiles - 1) / tiles);
+    if (want > n16) want = n16;
+    ConvPlan p;
+    for (int pass = 0; pass < 2; ++pass)   // two stages at least, by narrower chunks if need be; else one
+        for (int nch = want; nch <= n16; ++nch) {
+            p.Nc = (n16 + nch - 1) / nch * 16;
+            p.nchunks = (N + p.Nc - 1) / p.Nc;
+            if (pass == 0) {
+                const bool many = tiles * p.nchunks > sms;
+                if (many && conv_plan_try(p, K, parts, 9, true, 3, kConvStages, kSmemTwo)) return p;
+                if (many && conv_plan_try(p, K, parts, 9, true, 2, kConvStages, kSmemOne)) return p;
+                if (conv_plan_try(p, K, parts, 9, false, 2, kConvStages, kSmemOne)) return p;
+                if (conv_plan_try(p, K, parts, 3, false, 2, kConvStages, kSmemOne)) return p;
+            } else if (conv_plan_try(p, K, parts, 3, false, 1, 1, kSmemOne)) {
+                return p;
+            }
+        }
+    throw Error(UWGPU_ERR_ARGUMENT, "tensor-core kernel: shared memory plan too large");
 }
 
-// 3x3x3 convolution as an implicit GEMM on the tensor core: for a tile of 128 consecutive voxels
-// (rows, M = 128) and all N output channels, D = sum over the 27 taps t of A_t B_t^T, with
+// 3x3x3 convolution as an implicit GEMM on the tensor core: for a tile of 8 x 16 voxels (rows,
+// M = 128) and Nc output channels, D = sum over the 27 taps t of A_t B_t^T, with
 // A_t[m][k] = in[v_m + off(t)][k] (zero outside the grid) and B_t[n][k] = W_t[k][n], read from the
 // layer's other packing Wrev[26 - t][n][k] (for the forward pass the flipped transpose, for the
 // data gradient the plain weights).  Operands are K-major in shared memory; the accumulator
-// (128 x N FP32) lives in TMEM; one thread issues the MMAs of a tap while all threads stage the
-// next tap into the other buffer.  The epilogue adds the bias, applies ReLU and stores BF16 (or
-// FP32) rows.  CTAs are persistent over the voxel tiles.  FP32 inputs (gradients) enter as
-// hi + lo BF16 parts (two MMAs per K step).
-template <typename TI, typename TO>
-__global__ void __launch_bounds__(128, 1) k_conv3_tc(Vol g, int K, int N, ConvTcPlan P, const TI* __restrict__ in,
-                                                     const bf16* __restrict__ Wrev, const float* __restrict__ bias,
-                                                     TO* __restrict__ out, int relu, uint32_t* __restrict__ err) {
-    constexpr bool kSplit = sizeof(TI) == 4;
+// (128 x Nc FP32) lives in TMEM; one thread issues the MMAs of a stage while the next ones are
+// loaded.  The epilogue adds the bias, applies ReLU and stores BF16 (or FP32) rows.  CTAs are
+// persistent over the tiles of their channels.  A gradient comes as its hi and lo parts
+// (PARTS = 2, two MMAs per K step).  Every output element sums its taps and channels in the
+// same order whatever the plan, so its bits do not depend on it.
+//
+// Measured on the 16/32/64/128 network at 56 x 56 x 56 voxels, the 14 layers: forward 1158 -> 296 us, data
+// gradient 1631 -> 362 us against one voxel row per thread staged anew for each tap (bound by the latency
+// of those loads: a coarse layer's 3 or 22 tiles took 27 x 5 us on as many SMs).  At 16 channels a tile now
+// costs 2.3 us of an SM for 27 MMAs of 0.02 us: the staging's instructions bound it, which is why small
+// plans run with 128 threads (256: 41 us for a 16-channel layer, 128: 23 us); the coarse layers (9 to 36 us)
+// are bound by loading up to 390 KB of weights and halo per CTA.
+template <int PARTS, typename TO>
+__global__ void __launch_bounds__(kConvThreads, 2) k_conv3_tc(Vol g, int K, int N, ConvPlan P, const bf16* __restrict__ in,
+                                                           const bf16* __restrict__ in_lo, const bf16* __restrict__ Wrev,
+                                                           const float* __restrict__ bias, TO* __restrict__ out,
+                                                           int relu, uint32_t* __restrict__ err) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bar[kConvStages];
     __shared__ uint32_t tbase;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int Kp = P.Kp, Np = P.Np, kc8 = Kp / 8;
-    unsigned char* sB = smem;
-    unsigned char* sA = smem + (P.resident ? 27 : 2) * P.bytesB;   // [buf][part] of bytesA each
-    const uint32_t ncols = tc::tmem_cols(Np);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), threads = blockDim.x;
+    const int n0 = blockIdx.y * P.Nc, ahead = ring_ahead(P.stages);
+    const uint32_t ncols = tc::tmem_cols(P.Nc);
     if (warp == 0) {
         tc::tmem_alloc(&tbase, ncols);
         tc::tmem_relinquish();
     }
-    if (tid == 0) {
-        tc::mbar_init(&bar[0], 1);
-        tc::mbar_init(&bar[1], 1);
-    }
-    // B of tap t into `dst` (K-major, zero beyond N and K)
-    auto stage_b = [&](int t, unsigned char* dst) {
-        const bf16* src = Wrev + (size_t)(26 - t) * N * K;
-        for (int idx = tid; idx < Np * kc8; idx += 128) {
-            const int n = idx % Np, c8 = idx / Np;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (n < N && c8 * 8 < K) v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)n * K + c8 * 8));
-            *reinterpret_cast<uint4*>(dst + tc::k_major_offset(n, c8 * 8, Kp)) = v;
+    if (tid == 0)
+        for (int i = 0; i < P.stages; ++i) tc::mbar_init(&bar[i], 1);
+    const uint32_t sB = tc::smem_u32(smem), sA = sB + (P.resident ? 27u * P.tapB : 0u);
+    const int ntx = (g.px + kTx - 1) / kTx, nty = (g.py + kTy - 1) / kTy, nst = 27 / P.taps;
+    const int ntiles = ntx * nty * g.pz;
+    // weights of `count` taps from `t0`
+    auto load_b = [&](int t0, int count, uint32_t dst) {
+        const int rows = count * P.Nc;
+        for (int e = tid; e < rows * P.kc8; e += threads) {
+            const int row = e / P.kc8, c8 = e - row * P.kc8, tt = row / P.Nc, n = row - tt * P.Nc;
+            const bool live = n0 + n < N && c8 * 8 < K;
+            const bf16* src = live ? Wrev + ((int64_t)(26 - t0 - tt) * N + n0 + n) * K + c8 * 8 : Wrev;
+            cp_async16(dst + tt * P.tapB + c8 * P.chunkB + n * 16, src, live);
         }
     };
-    if (P.resident)
-        for (int t = 0; t < 27; ++t) stage_b(t, sB + (size_t)t * P.bytesB);
-    tc::fence_proxy_async();
+    // loader state: slot of the ring, stage of the tile, the tile and its first voxel
+    const int rowsA = (P.taps == 9 ? kTy + 2 : kTy) * kHx, kcK = K / 8;
+    const int step_r = threads / P.kc8, step_c = threads % P.kc8, row0 = tid / P.kc8, col0 = tid % P.kc8;
+    int l_slot = 0, l_s = 0, l_tile = blockIdx.x, l_x = 0, l_y = 0, l_z = 0;
+    auto load_stage = [&]() {
+        if (l_s == 0) {
+            const int t = l_tile / ntx;
+            l_x = (l_tile - t * ntx) * kTx - 1;
+            l_z = t / nty;
+            l_y = (t - l_z * nty) * kTy - 1;
+        }
+        const int s = l_s, z = l_z - 1 + (P.taps == 9 ? s : s / 3), y0 = l_y + (P.taps == 9 ? 0 : s % 3);
+        const int64_t base = ((int64_t)l_x + (int64_t)g.px * (y0 + (int64_t)g.py * z)) * K;
+        const uint32_t dst = sA + (uint32_t)l_slot * P.stage;
+        const unsigned py = z >= 0 && z < g.pz ? (unsigned)g.py : 0u;   // a plane outside the grid: no row is live
+        int row = row0, c8 = col0;
+        while (row < rowsA) {
+            const int yy = row / kHx, xx = row - yy * kHx;
+            const bool live = (unsigned)(l_x + xx) < (unsigned)g.px && (unsigned)(y0 + yy) < py && c8 < kcK;
+            const int64_t o = live ? base + ((yy * g.px + xx) * K + c8 * 8) : 0;
+            const uint32_t d = dst + c8 * P.chunkA + row * 16;
+            cp_async16(d, in + o, live);
+            if (PARTS == 2) cp_async16(d + P.partA, in_lo + o, live);
+            row += step_r;
+            c8 += step_c;
+            if (c8 >= P.kc8) {
+                c8 -= P.kc8;
+                ++row;
+            }
+        }
+        if (!P.resident) load_b(s * P.taps, P.taps, dst + PARTS * P.partA);
+        if (++l_slot == P.stages) l_slot = 0;
+        if (++l_s == nst) {
+            l_s = 0;
+            l_tile += gridDim.x;
+        }
+    };
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t taddr = tbase;
-    const uint32_t idesc = tc::idesc_f16(128, Np, tc::kFmtBF16, 0, 0);
-    uint32_t phase[2] = {0u, 0u}, pend[2] = {0u, 0u};
+    const uint32_t idesc = tc::idesc_f16(128, P.Nc, tc::kFmtBF16, 0, 0);
+    RingWait ring{bar, P.stages};
+    const int total = (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * nst : 0;
     bool ok = true;
-    auto wait_buf = [&](int b) {
-        if (pend[b]) {
-            ok = tc::mbar_wait(&bar[b], phase[b]) && ok;
-            phase[b] ^= 1u;
-            pend[b] = 0u;
+    if (P.resident) load_b(0, 27, sB);   // arrives with the first stage
+    for (int i = 0; i < ahead; ++i) {
+        if (i < total) load_stage();
+        cp_commit();
+    }
+    int i = 0, slot = 0, s = 0, tile = blockIdx.x;
+    for (; i < total; ++i) {
+        if (i + ahead < total) {
+            if (i + ahead >= P.stages) ok = ring.upto(i + ahead - P.stages) && ok;
+            load_stage();
         }
-    };
-    const int64_t ntiles = (g.nv + 127) / 128;
-    const int64_t pxy = (int64_t)g.px * g.py;
-    for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const int64_t v = tile * 128 + tid;   // this thread's row
-        const bool vin = v < g.nv;
-        const int x = (int)(v % g.px), y = (int)((v / g.px) % g.py), z = (int)(v / pxy);
-        for (int t = 0; t < 27; ++t) {
-            const int b = t & 1;
-            wait_buf(b);
-            unsigned char* a0 = sA + (size_t)b * (kSplit ? 2 : 1) * P.bytesA;
-            const int xx = x + t % 3 - 1, yy = y + (t / 3) % 3 - 1, zz = z + t / 9 - 1;
-            const bool nb = vin && xx >= 0 && xx < g.px && yy >= 0 && yy < g.py && zz >= 0 && zz < g.pz;
-            const TI* row = in + ((int64_t)xx + (int64_t)g.px * (yy + (int64_t)g.py * zz)) * K;
-            for (int c8 = 0; c8 < kc8; ++c8) {
-                const uint32_t off = tc::k_major_offset(tid, c8 * 8, Kp);
-                const bool live = nb && c8 * 8 < K;
-                if (kSplit) {
-                    uint4 hi = make_uint4(0, 0, 0, 0), lo = make_uint4(0, 0, 0, 0);
-                    if (live) split8(reinterpret_cast<const float*>(row) + c8 * 8, hi, lo);
-                    *reinterpret_cast<uint4*>(a0 + off) = hi;
-                    *reinterpret_cast<uint4*>(a0 + P.bytesA + off) = lo;
-                } else {
-                    uint4 val = make_uint4(0, 0, 0, 0);
-                    if (live) val = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(row) + c8 * 8));
-                    *reinterpret_cast<uint4*>(a0 + off) = val;
-                }
-            }
-            unsigned char* bt = P.resident ? sB + (size_t)t * P.bytesB : sB + (size_t)b * P.bytesB;
-            if (!P.resident) stage_b(t, bt);
-            tc::fence_proxy_async();
-            tc::fence_before_sync();
-            ok = __syncthreads_and(ok) != 0;
-            if (!ok) break;
-            tc::fence_after_sync();
-            if (tid == 0) {
-                const uint32_t sa = tc::smem_u32(a0), sb = tc::smem_u32(bt);
-                for (int s = 0; s < Kp / 16; ++s) {
-                    const uint64_t db = tc::k_major_desc(sb, s, Kp);
-                    tc::mma_f16(taddr, tc::k_major_desc(sa, s, Kp), db, idesc, (t > 0 || s > 0) ? 1u : 0u);
-                    if (kSplit) tc::mma_f16(taddr, tc::k_major_desc(sa + (uint32_t)P.bytesA, s, Kp), db, idesc, 1u);
-                }
-                tc::mma_commit(&bar[b]);
-            }
-            pend[b] = 1u;
-        }
-        wait_buf(0);
-        wait_buf(1);
+        cp_commit();
+        cp_wait(ahead);
+        tc::fence_proxy_async();
+        tc::fence_before_sync();
         ok = __syncthreads_and(ok) != 0;
         if (!ok) break;
         tc::fence_after_sync();
-        // epilogue: this thread's row, 16 columns at a time
-        for (int c = 0; c < Np; c += 16) {
+        if (warp == 0 && tc::elect_one()) {
+            const uint32_t a = sA + (uint32_t)slot * P.stage;
+            const uint32_t b = P.resident ? sB + (uint32_t)(s * P.taps) * P.tapB : a + PARTS * P.partA;
+            uint64_t da = tc::smem_desc(a, P.chunkA, kHx * 16u), db = tc::smem_desc(b, P.chunkB, 128u);
+            const uint64_t ka = 2u * P.chunkA >> 4, kb = 2u * P.chunkB >> 4, lo = P.partA >> 4, tb = P.tapB >> 4;
+            uint32_t acc = s > 0 ? 1u : 0u;
+            auto tap = [&](uint64_t ta) {   // addresses of a descriptor are in units of 16 bytes
+                uint64_t td = db;
+                for (int k = 0; k < P.kc8; k += 2, ta += ka, td += kb) {
+                    tc::mma_f16(taddr, ta, td, idesc, acc);
+                    acc = 1u;
+                    if (PARTS == 2) tc::mma_f16(taddr, ta + lo, td, idesc, 1u);
+                }
+                db += tb;
+            };
+            if (P.taps == 9) {
+#pragma unroll
+                for (int r = 0; r < 9; ++r) tap(da + (uint64_t)(r / 3 * kHx + r % 3));
+            } else {
+#pragma unroll
+                for (int r = 0; r < 3; ++r) tap(da + (uint64_t)r);
+            }
+            tc::mma_commit(&bar[slot]);
+        }
+        __syncwarp();
+        if (++slot == P.stages) slot = 0;
+        if (++s < nst) continue;
+        s = 0;
+        ok = ring.upto(i);
+        ok = __syncthreads_and(ok) != 0;
+        if (!ok) break;
+        tc::fence_after_sync();
+        // epilogue: this thread's row, 16 columns at a time, the two halves of the warps in turn
+        const int m = tid & 127;
+        const int tq = tile / ntx, z = tq / nty;
+        const int x = (tile - tq * ntx) * kTx + m % kTx, y = (tq - z * nty) * kTy + m / kTx;
+        tile += gridDim.x;
+        const bool vin = x < g.px && y < g.py;
+        const int64_t v = (int64_t)x + (int64_t)g.px * (y + (int64_t)g.py * z);
+        for (int c = 16 * (warp >> 2); c < P.Nc; c += threads >> 3) {
             uint32_t r[16];
-            tc::tmem_ld16(tc::tmem_addr(taddr, 32 * warp, c), r);
+            tc::tmem_ld16(tc::tmem_addr(taddr, 32 * (warp & 3), c), r);
             tc::tmem_wait_ld();
             if (!vin) continue;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int c0 = c + 8 * h;
+                const int c0 = n0 + c + 8 * h;
                 if (c0 >= N) break;
                 float o[8];
 #pragma unroll
@@ -229,11 +352,11 @@ __global__ void __launch_bounds__(128, 1) k_conv3_tc(Vol g, int K, int N, ConvTc
         __syncthreads();
         tc::fence_after_sync();
     }
+    cp_wait(0);
     if (!ok) {
         if (tid == 0) atomicOr(err, 1u);
         // give MMAs still in flight a bounded time to finish before the TMEM is released
-        for (int b = 0; b < 2; ++b)
-            if (pend[b]) tc::mbar_wait(&bar[b], phase[b], 1u << 16);
+        ring.upto(i - 1, 1u << 16);
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -243,117 +366,191 @@ __global__ void __launch_bounds__(128, 1) k_conv3_tc(Vol g, int K, int N, ConvTc
     }
 }
 
-// Weight gradient on the tensor core: part[slice][t][ci][co] = sum over the slice's voxels v of
-// in[v + off(t)][ci] g[v][co].  Rows M are the (tap, input channel) pairs, 128 per CTA (grid.x);
-// N the output channels; K the voxels, 64 per stage, double-buffered.  Both operands are
-// MN-major in shared memory: a 16-byte chunk holds 8 consecutive channels of one voxel, as the
-// channels-last tensors store them.  The FP32 gradient enters as hi + lo BF16 parts.  Each CTA
-// (grid.y) owns a fixed voxel slice, and the slices are summed in a fixed order afterwards, so the
-// gradient is deterministic.
-constexpr int kWgK = 64;   // voxels per stage
-__host__ __device__ inline size_t wgrad_tc_smem(int Np) {
-    return 2 * ((size_t)128 * kWgK * 2 + 2 * (size_t)Np * kWgK * 2);
+// Plan of k_conv3_wgrad_tc.  A CTA owns `taps` taps (27, 9 or 3), `nci` input and `cw` output
+// channels: taps * Np accumulator columns, 512 at most.
+struct WgradPlan {
+    int ty, ntx, nty;    // rows in y of a tile (even), tiles in x and y
+    int taps, groups;    // taps of a CTA, groups of taps
+    int nci, Np, nchunk; // input channels of a CTA (padded to 16: Np), chunks of them
+    int cw, nco;         // output channels of a CTA (64 at most: hi and lo rows make M = 128), chunks of them
+    int stages, planes;
+    int ntiles, per;     // voxel tiles, tiles per slice
+    uint32_t chunkI, planeI, chunkG, stage;
+    size_t smem;
+};
+inline WgradPlan wgrad_plan(const Vol& g, int cin, int cout) {
+    WgradPlan p;
+    p.ntx = (g.px + kTx - 1) / kTx;
+    p.nty = (g.py + kTy - 1) / kTy;
+    p.ty = ((g.py + p.nty - 1) / p.nty + 1) / 2 * 2;
+    p.ntiles = p.ntx * p.nty * g.pz;
+    p.nchunk = cin <= 160 ? 1 : (cin + 127) / 128;
+    p.nci = ((cin + p.nchunk - 1) / p.nchunk + 7) / 8 * 8;
+    p.Np = (p.nci + 15) / 16 * 16;
+    p.taps = 27 * p.Np <= 512 ? 27 : 9 * p.Np <= 512 ? 9 : 3;
+    p.groups = 27 / p.taps;
+    p.planes = p.taps == 27 ? 3 : 1;
+    p.cw = cout < 64 ? cout : 64;
+    p.nco = (cout + 63) / 64;
+    p.chunkI = (uint32_t)chunk_rows((p.taps == 3 ? p.ty : p.ty + 2) * kHx, p.Np / 8) * 16u;
+    p.planeI = (uint32_t)(p.Np / 8) * p.chunkI;
+    p.chunkG = (uint32_t)chunk_rows(p.ty * kTx, p.cw / 8) * 16u;
+    p.stage = (uint32_t)p.planes * p.planeI + 16u * p.chunkG;
+    const int fit = (int)(kSmemOne / p.stage);
+    p.stages = fit < kConvStages ? fit : kConvStages;
+    p.smem = (size_t)p.stages * p.stage;
+    return p;
 }
-__global__ void __launch_bounds__(128, 1) k_conv3_wgrad_tc(Vol g, int cin, int cout, int Np, int64_t vslice,
-                                                           const bf16* __restrict__ in, const float* __restrict__ gout,
-                                                           float* __restrict__ part, uint32_t* __restrict__ err) {
+
+// Weight gradient on the tensor core: part[slice][hi, lo][t][ci][co] = sum over the slice's voxels
+// v of in[v + off(t)][ci] g[v][co].  M = 128 rows hold the output channels of the gradient's hi
+// part and then of its lo part, N the input channels, one accumulator per tap, K the voxels of a
+// tile, two rows in y (16 voxels) per MMA.  Both operands are MN-major: a 16-byte chunk holds 8
+// consecutive channels of one voxel, as the channels-last tensors store them; the input of a tap
+// is the staged halo at a shifted start address.  Each CTA (grid.y) owns a fixed slice of the
+// tiles, and the slices are summed in a fixed order afterwards, so the gradient is deterministic.
+// Rows of channels that do not exist multiply whatever the shared memory holds and are not read.
+//
+// Measured on the same network, the 14 layers: 1981 -> 470 us against rows of (tap, input channel) gathered
+// for each group of 128 (27 readings of the input, the gradient split into parts in each).  Bound by the MMA
+// count at few channels: 0.03 us per MMA of 128 x 16 x 16, of whose 128 rows 16 output channels use 32.
+__global__ void __launch_bounds__(kConvThreads, 2) k_conv3_wgrad_tc(Vol g, int cin, int cout, WgradPlan P,
+                                                                 const bf16* __restrict__ in,
+                                                                 const bf16* __restrict__ g_hi,
+                                                                 const bf16* __restrict__ g_lo,
+                                                                 float* __restrict__ part, uint32_t* __restrict__ err) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bar[kConvStages];
     __shared__ uint32_t tbase;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int rows = 27 * cin;
-    const int r0 = blockIdx.x * 128;
-    const size_t bytesA = (size_t)128 * kWgK * 2, bytesB = (size_t)Np * kWgK * 2;
-    const size_t stage_bytes = bytesA + 2 * bytesB;
-    const uint32_t ncols = tc::tmem_cols(Np);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), ahead = ring_ahead(P.stages);
+    const int grp = blockIdx.x % P.groups, chunk = blockIdx.x / P.groups % P.nchunk;
+    const int co0 = blockIdx.x / (P.groups * P.nchunk) * 64, ci0 = chunk * P.nci;
+    const int ci1 = ci0 + P.nci < cin ? ci0 + P.nci : cin;
+    const uint32_t ncols = tc::tmem_cols(P.taps * P.Np);
     if (warp == 0) {
         tc::tmem_alloc(&tbase, ncols);
         tc::tmem_relinquish();
     }
-    if (tid == 0) {
-        tc::mbar_init(&bar[0], 1);
-        tc::mbar_init(&bar[1], 1);
-    }
+    if (tid == 0)
+        for (int i = 0; i < P.stages; ++i) tc::mbar_init(&bar[i], 1);
+    const uint32_t s0 = tc::smem_u32(smem);
+    const int first = (int)blockIdx.y * P.per;
+    const int total = first + P.per < P.ntiles ? P.per : P.ntiles - first;
+    const int kc8 = P.Np / 8, rowsI = (P.taps == 3 ? P.ty : P.ty + 2) * kHx;
+    const int gc8 = P.cw / 8, rowsG = P.ty * kTx;
+    const int irow = tid / kc8, icol = tid % kc8, istep_r = kConvThreads / kc8, istep_c = kConvThreads % kc8;
+    const int grow = tid / gc8, gcol = tid % gc8, gstep_r = kConvThreads / gc8, gstep_c = kConvThreads % gc8;
+    const int ilive = (ci1 - ci0) / 8, glive = (cout - co0) / 8;   // chunks that exist
+    int l_slot = 0, l_tile = first;
+    auto load_stage = [&]() {
+        const int tq = l_tile / P.ntx, z0 = tq / P.nty;
+        const int x0 = (l_tile - tq * P.ntx) * kTx, y0 = (tq - z0 * P.nty) * P.ty;
+        const uint32_t dst = s0 + (uint32_t)l_slot * P.stage;
+        const int ya = y0 - 1 + (P.taps == 3 ? grp % 3 : 0);
+        for (int pl = 0; pl < P.planes; ++pl) {
+            const int z = z0 - 1 + (P.taps == 27 ? pl : P.taps == 9 ? grp : grp / 3);
+            const unsigned py = z >= 0 && z < g.pz ? (unsigned)g.py : 0u;   // a plane outside the grid: no row is live
+            const int64_t base = ((int64_t)(x0 - 1) + (int64_t)g.px * (ya + (int64_t)g.py * z)) * cin + ci0;
+            int row = irow, c8 = icol;
+            while (row < rowsI) {
+                const int yy = row / kHx, xx = row - yy * kHx;
+                const bool live = (unsigned)(x0 - 1 + xx) < (unsigned)g.px && (unsigned)(ya + yy) < py && c8 < ilive;
+                const int64_t o = live ? base + ((yy * g.px + xx) * cin + c8 * 8) : 0;
+                cp_async16(dst + pl * P.planeI + c8 * P.chunkI + row * 16, in + o, live);
+                row += istep_r;
+                c8 += istep_c;
+                if (c8 >= kc8) {
+                    c8 -= kc8;
+                    ++row;
+                }
+            }
+        }
+        const uint32_t dg = dst + P.planes * P.planeI;
+        const int64_t base = ((int64_t)x0 + (int64_t)g.px * (y0 + (int64_t)g.py * z0)) * cout + co0;
+        int k = grow, c8 = gcol;
+        while (k < rowsG) {
+            const int xx = k % kTx, yy = k / kTx;
+            const bool live = x0 + xx < g.px && y0 + yy < g.py && c8 < glive;
+            const int64_t o = live ? base + ((yy * g.px + xx) * cout + c8 * 8) : 0;
+            const uint32_t d = dg + c8 * P.chunkG + k * 16;
+            cp_async16(d, g_hi + o, live);
+            cp_async16(d + gc8 * P.chunkG, g_lo + o, live);
+            k += gstep_r;
+            c8 += gstep_c;
+            if (c8 >= gc8) {
+                c8 -= gc8;
+                ++k;
+            }
+        }
+        ++l_tile;
+        if (++l_slot == P.stages) l_slot = 0;
+    };
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t taddr = tbase;
-    const uint32_t idesc = tc::idesc_f16(128, Np, tc::kFmtBF16, 1, 1);
-    const int64_t v0 = (int64_t)blockIdx.y * vslice;
-    const int64_t v1 = v0 + vslice < g.nv ? v0 + vslice : g.nv;
-    const int64_t pxy = (int64_t)g.px * g.py;
-    uint32_t phase[2] = {0u, 0u}, pend[2] = {0u, 0u};
+    const uint32_t idesc = tc::idesc_f16(128, P.Np, tc::kFmtBF16, 1, 1);
+    RingWait ring{bar, P.stages};
     bool ok = true;
-    int step = 0;
-    for (int64_t vb = v0; vb < v1; vb += kWgK, ++step) {
-        const int b = step & 1;
-        if (pend[b]) {
-            ok = tc::mbar_wait(&bar[b], phase[b]) && ok;
-            phase[b] ^= 1u;
-            pend[b] = 0u;
+    for (int i = 0; i < ahead; ++i) {
+        if (i < total) load_stage();
+        cp_commit();
+    }
+    int i = 0, slot = 0;
+    for (; i < total; ++i) {
+        if (i + ahead < total) {
+            if (i + ahead >= P.stages) ok = ring.upto(i + ahead - P.stages) && ok;
+            load_stage();
         }
-        unsigned char* sa = smem + (size_t)b * stage_bytes;
-        unsigned char* sbh = sa + bytesA;
-        unsigned char* sbl = sbh + bytesB;
-        // A: 16 row groups (8 channels of one tap) x 64 voxels
-        for (int idx = tid; idx < 16 * kWgK; idx += 128) {
-            const int k = idx % kWgK, mg = idx / kWgK;   // consecutive threads: consecutive voxels
-            const int r = r0 + mg * 8;
-            const int64_t v = vb + k;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (r < rows && v < v1) {
-                const int t = r / cin, ci = r % cin;
-                const int x = (int)(v % g.px) + t % 3 - 1, y = (int)((v / g.px) % g.py) + (t / 3) % 3 - 1,
-                          z = (int)(v / pxy) + t / 9 - 1;
-                if (x >= 0 && x < g.px && y >= 0 && y < g.py && z >= 0 && z < g.pz)
-                    val = __ldg(reinterpret_cast<const uint4*>(in + ((int64_t)x + (int64_t)g.px * (y + (int64_t)g.py * z)) * cin + ci));
-            }
-            *reinterpret_cast<uint4*>(sa + tc::mn_major_offset(mg * 8, k, 128)) = val;
-        }
-        // B: Np / 8 groups of output channels x 64 voxels, hi and lo parts
-        for (int idx = tid; idx < (Np / 8) * kWgK; idx += 128) {
-            const int k = idx % kWgK, ng = idx / kWgK;
-            const int64_t v = vb + k;
-            uint4 hi = make_uint4(0, 0, 0, 0), lo = make_uint4(0, 0, 0, 0);
-            if (ng * 8 < cout && v < v1) split8(gout + v * cout + ng * 8, hi, lo);
-            const uint32_t off = tc::mn_major_offset(ng * 8, k, Np);
-            *reinterpret_cast<uint4*>(sbh + off) = hi;
-            *reinterpret_cast<uint4*>(sbl + off) = lo;
-        }
+        cp_commit();
+        cp_wait(ahead);
         tc::fence_proxy_async();
         tc::fence_before_sync();
         ok = __syncthreads_and(ok) != 0;
         if (!ok) break;
         tc::fence_after_sync();
-        if (tid == 0) {
-            const uint32_t a = tc::smem_u32(sa), bh = tc::smem_u32(sbh), bl = tc::smem_u32(sbl);
-            for (int s = 0; s < kWgK / 16; ++s) {
-                const uint64_t da = tc::mn_major_desc(a, s, 128);
-                tc::mma_f16(taddr, da, tc::mn_major_desc(bh, s, Np), idesc, (step > 0 || s > 0) ? 1u : 0u);
-                tc::mma_f16(taddr, da, tc::mn_major_desc(bl, s, Np), idesc, 1u);
+        if (warp == 0 && tc::elect_one()) {
+            const uint32_t a = s0 + (uint32_t)slot * P.stage;
+            uint64_t da = tc::smem_desc(a + P.planes * P.planeI, 128u, P.chunkG);
+            uint64_t db = tc::smem_desc(a, kHx * 16u, P.chunkI);
+            for (int ks = 0; ks < P.ty / 2; ++ks) {   // addresses of a descriptor are in units of 16 bytes
+                const uint32_t acc = (i > 0 || ks > 0) ? 1u : 0u;
+                uint32_t d = taddr;
+                if (P.taps == 3) {
+#pragma unroll
+                    for (int r = 0; r < 3; ++r, d += P.Np) tc::mma_f16(d, da, db + (uint64_t)r, idesc, acc);
+                } else {
+                    uint64_t dp = db;
+                    for (int pl = 0; pl < P.planes; ++pl, dp += P.planeI >> 4) {
+#pragma unroll
+                        for (int r = 0; r < 9; ++r, d += P.Np)
+                            tc::mma_f16(d, da, dp + (uint64_t)(r / 3 * kHx + r % 3), idesc, acc);
+                    }
+                }
+                da += 16u;
+                db += 2u * kHx;
             }
-            tc::mma_commit(&bar[b]);
+            tc::mma_commit(&bar[slot]);
         }
-        pend[b] = 1u;
+        __syncwarp();
+        if (++slot == P.stages) slot = 0;
     }
-    for (int b = 0; b < 2; ++b)
-        if (pend[b]) {
-            ok = tc::mbar_wait(&bar[b], phase[b]) && ok;
-            phase[b] ^= 1u;
-            pend[b] = 0u;
-        }
+    cp_wait(0);
+    // every MMA issued (after a failure: bounded time to finish before the TMEM is released)
+    ok = ring.upto(i - 1, ok ? 1u << 22 : 1u << 16) && ok;
     ok = __syncthreads_and(ok) != 0;
     tc::fence_after_sync();
-    const int r = r0 + tid;
-    float* dst = part + ((int64_t)blockIdx.y * rows + r) * cout;
-    for (int c = 0; c < Np && ok; c += 16) {
+    const int m = tid & 127, cwr = gc8 * 8, p = m / cwr, co = co0 + m % cwr;
+    for (int c = 16 * (warp >> 2); c < P.taps * P.Np && ok && 32 * (warp & 3) < 2 * cwr; c += 32) {
         uint32_t v[16];
-        tc::tmem_ld16(tc::tmem_addr(taddr, 32 * warp, c), v);
+        tc::tmem_ld16(tc::tmem_addr(taddr, 32 * (warp & 3), c), v);
         tc::tmem_wait_ld();
-        if (r >= rows) continue;
+        if (p > 1 || co >= cout) continue;
+        const int t = grp * P.taps + c / P.Np, ci = ci0 + c % P.Np;
+        float* dst = part + ((((int64_t)blockIdx.y * 2 + p) * 27 + t) * cin + ci) * cout + co;
 #pragma unroll
         for (int j = 0; j < 16; ++j)
-            if (c + j < cout) dst[c + j] = step > 0 ? __uint_as_float(v[j]) : 0.0f;
+            if (ci + j < ci1) dst[(int64_t)j * cout] = __uint_as_float(v[j]);
     }
     if (!ok && tid == 0) atomicOr(err, 1u);
     tc::fence_before_sync();
@@ -364,13 +561,27 @@ __global__ void __launch_bounds__(128, 1) k_conv3_wgrad_tc(Vol g, int cin, int c
     }
 }
 
-// dst[i] += sum_s part[s][i], s ascending
-__global__ void k_sum_slices(int64_t n, int slices, const float* __restrict__ part, float* __restrict__ dst) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// sum of `slices` values `n` apart, ascending, sixteen loads in flight
+__device__ __forceinline__ float ordered_sum(const float* __restrict__ p, int64_t n, int slices) {
     float a = 0.0f;
-    for (int sl = 0; sl < slices; ++sl) a += part[(int64_t)sl * n + i];
-    dst[i] += a;
+    int sl = 0;
+    for (; sl + 16 <= slices; sl += 16, p += 16 * n) {
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = __ldg(p + k * n);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) a += v[k];
+    }
+    for (; sl < slices; ++sl, p += n) a += __ldg(p);
+    return a;
+}
+// dst[i] += sum_s part[s][i], s ascending: n1 values of `slices1` slices and behind them n2 of `slices2`
+// slices of part2 (a layer's weights and its biases, adjacent in the parameter vector)
+__global__ void k_sum_slices(int64_t n1, int slices1, const float* __restrict__ part, int n2, int slices2,
+                             const float* __restrict__ part2, float* __restrict__ dst) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n1 + n2) return;
+    dst[i] += i < n1 ? ordered_sum(part + i, n1, slices1) : ordered_sum(part2 + (i - n1), n2, slices2);
 }
 
 // part[block][co] = sum over the block's voxels of g[v][co] (thread t covers channel t % cout of
@@ -390,10 +601,24 @@ __global__ void k_bias_grad(int64_t nv, int cout, const float* __restrict__ gout
     }
 }
 
-// g = g * (y > 0): gradient through ReLU, y the stored BF16 output of the layer
-__global__ void k_relu_bwd(int64_t n, const bf16* __restrict__ y, float* __restrict__ g) {
+// g = g * (y > 0): gradient through ReLU, y the stored BF16 output of the layer, and the BF16 parts of g for
+// the layer's two gradient kernels (split here once: the kernels would split each value per tap and tile);
+// eight values per thread, n8 = values / 8
+__global__ void k_relu_bwd(int64_t n8, const bf16* __restrict__ y, float* __restrict__ g, bf16* __restrict__ hi,
+                           bf16* __restrict__ lo) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && !(__bfloat162float(y[i]) > 0.0f)) g[i] = 0.0f;
+    if (i >= n8) return;
+    float yv[8], gv[8];
+    load8(y + 8 * i, yv);
+    load8(g + 8 * i, gv);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (!(yv[k] > 0.0f)) gv[k] = 0.0f;
+    store8(g + 8 * i, gv);
+    uint4 h, l;
+    split8(gv, h, l);
+    reinterpret_cast<uint4*>(hi)[i] = h;
+    reinterpret_cast<uint4*>(lo)[i] = l;
 }
 
 // 2x2x2 average pooling (fine -> coarse), BF16
@@ -423,21 +648,24 @@ __global__ void k_pool_bwd_add(Vol f, Vol c, int ch, const float* __restrict__ g
     gf[i] += 0.125f * gc[V * ch + cc];
 }
 
-// decoder input: out[v] = [ up(coarse)[v] (cu channels) | skip[v] (cs channels) ]
+// decoder input: out[v] = [ up(coarse)[v] (cu channels) | skip[v] (cs channels) ], eight channels per thread
 __global__ void k_up_concat(Vol f, Vol c, int cu, int cs, const bf16* __restrict__ coarse,
                             const bf16* __restrict__ skip, bf16* __restrict__ out) {
-    const int ct = cu + cs;
+    const int ct8 = (cu + cs) / 8;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= f.nv * ct) return;
-    const int64_t v = i / ct;
-    const int cc = (int)(i % ct);
+    if (i >= f.nv * ct8) return;
+    const int64_t v = i / ct8;
+    const int cc = (int)(i - v * ct8) * 8;
+    const bf16* src;
     if (cc < cu) {
-        const int x = (int)(v % f.px), y = (int)((v / f.px) % f.py), z = (int)(v / ((int64_t)f.px * f.py));
+        const int64_t row = v / f.px;
+        const int x = (int)(v - row * f.px), z = (int)(row / f.py), y = (int)(row - (int64_t)z * f.py);
         const int64_t V = (x / 2) + (int64_t)c.px * ((y / 2) + (int64_t)c.py * (z / 2));
-        out[i] = coarse[V * cu + cc];
+        src = coarse + V * cu + cc;
     } else {
-        out[i] = skip[v * cs + (cc - cu)];
+        src = skip + v * cs + (cc - cu);
     }
+    reinterpret_cast<uint4*>(out)[i] = __ldg(reinterpret_cast<const uint4*>(src));
 }
 
 // gradient of k_up_concat: gc[V][c] = sum over the 8 children of g[v][c] (c < cu);
@@ -581,67 +809,68 @@ void check_errors(Context& c, Net& n) {
     }
 }
 
-// 3x3x3 convolution on the tensor core (k_conv3_tc).  W: the layer's weights as the convolution
-// reads them ([27][K][N]); Wrev: the layer's other packing ([27][N][K] in reverse tap order).
-template <typename TI, typename TO>
-static void conv_launch_tc(Context& c, Net& n, const Vol& g, int K, int N, const TI* in, const bf16* Wrev,
-                           const float* bias, TO* out, bool relu) {
-    const ConvTcPlan P = conv_tc_plan(K, N, sizeof(TI) == 4);
-    UWG_REQUIRE(P.Np <= 256, UWGPU_ERR_ARGUMENT, "U-Net layer too wide for the tensor-core convolution");
+// 3x3x3 convolution on the tensor core (k_conv3_tc).  Wrev: the layer's packing with the output channel
+// before the input channel, [27][N][K] in reverse tap order.  The widths accepted are those of which one
+// tap's weights and 128 voxels' inputs fit a CTA's shared memory twice.
+template <int PARTS, typename TO>
+static void conv_launch_tc(Context& c, Net& n, const Vol& g, int K, int N, const bf16* in, const bf16* in_lo,
+                           const bf16* Wrev, const float* bias, TO* out, bool relu) {
+    const int Kp = (K + 15) / 16 * 16, Np = (N + 15) / 16 * 16;
+    UWG_REQUIRE(Np <= 256, UWGPU_ERR_ARGUMENT, "U-Net layer too wide for the tensor-core convolution");
+    UWG_REQUIRE((size_t)4 * Kp * (Np + PARTS * 128) <= kSmemWidth, UWGPU_ERR_ARGUMENT,
+                "tensor-core kernel: shared memory plan too large");
+    const int64_t ntiles = (int64_t)((g.px + kTx - 1) / kTx) * ((g.py + kTy - 1) / kTy) * g.pz;
+    const int sms = sm_count(c);
+    const ConvPlan P = conv_plan(K, N, PARTS, ntiles, sms);
     int per_sm = 1;
     const size_t smem =
-        tmem_safe_smem((const void*)k_conv3_tc<TI, TO>, c.device, P.smem, tc::tmem_cols(P.Np), &per_sm);
-    const int64_t ntiles = (g.nv + 127) / 128;
-    const int64_t cap = (int64_t)sm_count(c) * per_sm;
-    const unsigned grid = (unsigned)(ntiles < cap ? ntiles : cap);
+        tmem_safe_smem((const void*)k_conv3_tc<PARTS, TO>, c.device, P.smem, tc::tmem_cols(P.Nc), &per_sm);
+    const int threads = P.smem <= kSmemTwo ? 128 : kConvThreads;
+    if (per_sm > 2048 / threads) per_sm = 2048 / threads;
+    const int64_t cap = std::max<int64_t>((int64_t)sms * per_sm / P.nchunks, 1);
+    const dim3 grid((unsigned)(ntiles < cap ? ntiles : cap), (unsigned)P.nchunks);
     LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
-    k_conv3_tc<TI, TO><<<grid, 128, smem, c.stream>>>(g, K, N, P, in, Wrev, bias, out, relu ? 1 : 0, n.tc_err.p);
-    note_work(c, UWGPU_KERNEL_LEARNED, (double)g.nv * (K * sizeof(TI) + N * sizeof(TO)),
-              2.0 * 27.0 * K * N * (double)g.nv * (sizeof(TI) == 4 ? 2.0 : 1.0));
+    k_conv3_tc<PARTS, TO><<<grid, threads, smem, c.stream>>>(g, K, N, P, in, in_lo, Wrev, bias, out, relu ? 1 : 0,
+                                                                  n.tc_err.p);
+    note_work(c, UWGPU_KERNEL_LEARNED, (double)g.nv * (K * PARTS * sizeof(bf16) + N * sizeof(TO)),
+              2.0 * 27.0 * K * N * (double)g.nv * PARTS);
 }
 
+// dW += the weight gradient from the layer's input and the parts (n.g_hi, n.g_lo) of its output gradient
+// gout; db (behind dW in the parameter vector) += the sums of gout
 static void wgrad_launch_tc(Context& c, Net& n, const Vol& g, int cin, int cout, const bf16* in, const float* gout,
                             float* dW, DArray<float>& part) {
-    const int Np = (cout + 15) / 16 * 16;
-    UWG_REQUIRE(Np <= 256, UWGPU_ERR_ARGUMENT, "U-Net layer too wide for the tensor-core weight gradient");
+    constexpr int kBiasBlocks = 152;
+    UWG_REQUIRE(cout <= 256, UWGPU_ERR_ARGUMENT, "U-Net layer too wide for the tensor-core weight gradient");
+    WgradPlan P = wgrad_plan(g, cin, cout);
     int per_sm = 1;
     const size_t smem =
-        tmem_safe_smem((const void*)k_conv3_wgrad_tc, c.device, wgrad_tc_smem(Np), tc::tmem_cols(Np), &per_sm);
-    const int rows = 27 * cin;
-    const int mtiles = (rows + 127) / 128;
-    int64_t slices = (2LL * sm_count(c) + mtiles - 1) / mtiles;
-    const int64_t max_slices = (g.nv + 511) / 512;
-    if (slices > max_slices) slices = max_slices;
-    if (slices < 1) slices = 1;
-    int64_t vslice = (g.nv + slices - 1) / slices;
-    vslice = (vslice + kWgK - 1) / kWgK * kWgK;
-    slices = (g.nv + vslice - 1) / vslice;
-    const int64_t nw = (int64_t)rows * cout;
-    part.ensure((size_t)slices * nw);
+        tmem_safe_smem((const void*)k_conv3_wgrad_tc, c.device, P.smem, tc::tmem_cols(P.taps * P.Np), &per_sm);
+    const int gx = P.groups * P.nchunk * P.nco;
+    int slices = std::max(sm_count(c) * per_sm / gx, 1);
+    if (slices > P.ntiles) slices = P.ntiles;
+    P.per = (P.ntiles + slices - 1) / slices;
+    slices = (P.ntiles + P.per - 1) / P.per;
+    const int64_t nw = (int64_t)27 * cin * cout;
+    part.ensure((size_t)slices * 2 * nw + (size_t)kBiasBlocks * cout);
+    float* bias_part = part.p + (size_t)slices * 2 * nw;
     {
         LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
-        k_conv3_wgrad_tc<<<dim3(mtiles, (unsigned)slices), 128, smem, c.stream>>>(g, cin, cout, Np, vslice, in, gout,
-                                                                                 part.p, n.tc_err.p);
+        k_bias_grad<<<kBiasBlocks, (256 / cout) * cout, 0, c.stream>>>(g.nv, cout, gout, bias_part);
+    }
+    {
+        LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
+        k_conv3_wgrad_tc<<<dim3(gx, (unsigned)slices), kConvThreads, smem, c.stream>>>(g, cin, cout, P, in, n.g_hi.p,
+                                                                                      n.g_lo.p, part.p, n.tc_err.p);
     }
     LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
-    k_sum_slices<<<nblk(nw, 256), 256, 0, c.stream>>>(nw, (int)slices, part.p, dW);
+    k_sum_slices<<<nblk(nw + cout, 256), 256, 0, c.stream>>>(nw, 2 * slices, part.p, cout, kBiasBlocks, bias_part, dW);
     note_work(c, UWGPU_KERNEL_LEARNED, (double)g.nv * 27.0 * (cin * 2 + cout * 4), 4.0 * 27.0 * cin * cout * (double)g.nv);
 }
 
-static void bias_grad_launch(Context& c, int64_t nv, int cout, const float* gout, float* db, DArray<float>& part) {
-    const int blocks = 152;
-    part.ensure((size_t)blocks * cout);
-    {
-        LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
-        k_bias_grad<<<blocks, (256 / cout) * cout, 0, c.stream>>>(nv, cout, gout, part.p);
-    }
+static void relu_bwd(Context& c, Net& n, int64_t count, const bf16* y, float* g) {
     LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
-    k_sum_slices<<<nblk(cout, 256), 256, 0, c.stream>>>(cout, blocks, part.p, db);
-}
-
-static void relu_bwd(Context& c, int64_t n, const bf16* y, float* g) {
-    LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
-    k_relu_bwd<<<nblk(n, 256), 256, 0, c.stream>>>(n, y, g);
+    k_relu_bwd<<<nblk(count / 8, 256), 256, 0, c.stream>>>(count / 8, y, g, n.g_hi.p, n.g_lo.p);
 }
 
 // splitmix64 (Steele, Lea and Flood 2014) for reproducible initial weights
@@ -733,6 +962,8 @@ void create(Context& c, Net& n, int levels, int base, uint64_t seed) {
     for (int l = 0; l < levels; ++l) {
         const int64_t nv = n.vol[l].nv;
         const int C = n.ch[l];
+        n.g_hi.ensure((size_t)nv * C);
+        n.g_lo.ensure((size_t)nv * C);
         n.enc_a[l].ensure((size_t)nv * C);
         n.enc_b[l].ensure((size_t)nv * C);
         n.g_enc_a[l].ensure((size_t)nv * C);
@@ -774,9 +1005,9 @@ void forward(Context& c, Net& n) {
         const Conv& a = n.convs[n.enc(l, 0)];
         const Conv& b = n.convs[n.enc(l, 1)];
         const bf16* in = l == 0 ? n.x0.p : n.pool[l - 1].p;
-        conv_launch_tc<bf16, bf16>(c, n, g, a.cin, a.cout, in, a.wflip.p, n.params.p + a.b_off, n.enc_a[l].p, true);
-        conv_launch_tc<bf16, bf16>(c, n, g, b.cin, b.cout, n.enc_a[l].p, b.wflip.p, n.params.p + b.b_off, n.enc_b[l].p,
-                                   true);
+        conv_launch_tc<1, bf16>(c, n, g, a.cin, a.cout, in, nullptr, a.wflip.p, n.params.p + a.b_off, n.enc_a[l].p, true);
+        conv_launch_tc<1, bf16>(c, n, g, b.cin, b.cout, n.enc_a[l].p, nullptr, b.wflip.p, n.params.p + b.b_off,
+                                n.enc_b[l].p, true);
         if (l + 1 < L) {
             const int64_t cnt = n.vol[l + 1].nv * n.ch[l];
             LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
@@ -788,17 +1019,17 @@ void forward(Context& c, Net& n) {
         const int cu = n.ch[l + 1], cs = n.ch[l];
         const bf16* coarse = l == L - 2 ? n.enc_b[L - 1].p : n.dec_b[l + 1].p;
         {
-            const int64_t cnt = g.nv * (cu + cs);
+            const int64_t cnt = g.nv * ((cu + cs) / 8);
             LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
             k_up_concat<<<nblk(cnt, 256), 256, 0, c.stream>>>(g, n.vol[l + 1], cu, cs, coarse, n.enc_b[l].p,
                                                               n.dec_cat[l].p);
         }
         const Conv& a = n.convs[n.dec(l, 0)];
         const Conv& b = n.convs[n.dec(l, 1)];
-        conv_launch_tc<bf16, bf16>(c, n, g, a.cin, a.cout, n.dec_cat[l].p, a.wflip.p, n.params.p + a.b_off, n.dec_a[l].p,
-                                   true);
-        conv_launch_tc<bf16, bf16>(c, n, g, b.cin, b.cout, n.dec_a[l].p, b.wflip.p, n.params.p + b.b_off, n.dec_b[l].p,
-                                   true);
+        conv_launch_tc<1, bf16>(c, n, g, a.cin, a.cout, n.dec_cat[l].p, nullptr, a.wflip.p, n.params.p + a.b_off,
+                                n.dec_a[l].p, true);
+        conv_launch_tc<1, bf16>(c, n, g, b.cin, b.cout, n.dec_a[l].p, nullptr, b.wflip.p, n.params.p + b.b_off,
+                                n.dec_b[l].p, true);
     }
     const bf16* fin = L == 1 ? n.enc_b[0].p : n.dec_b[0].p;
     {
@@ -809,15 +1040,14 @@ void forward(Context& c, Net& n) {
     check_launch("unet forward");
 }
 
-// gradient of one conv layer: g (pre-activation gradient, FP32, [nv][cout]) -> dW, db, and the
-// gradient of its input (post-activation of the layer below) into gin
+// gradient of one conv layer: g (pre-activation gradient, FP32, [nv][cout], its parts in n.g_hi and n.g_lo)
+// -> dW, db, and the gradient of its input (post-activation of the layer below) into gin
 static void conv_backward(Context& c, Net& n, const Vol& g, const Conv& cv, const bf16* in, const float* gpre,
                           float* gin) {
     wgrad_launch_tc(c, n, g, cv.cin, cv.cout, in, gpre, n.grads.p + cv.w_off, n.part);
-    bias_grad_launch(c, g.nv, cv.cout, gpre, n.grads.p + cv.b_off, n.part);
     // the data gradient is the convolution with W'[t][co][ci] = W[26 - t][ci][co]; its other
     // packing, read in reverse tap order, is the plain W
-    conv_launch_tc<float, float>(c, n, g, cv.cout, cv.cin, gpre, cv.w16.p, nullptr, gin, false);
+    conv_launch_tc<2, float>(c, n, g, cv.cout, cv.cin, n.g_hi.p, n.g_lo.p, cv.w16.p, nullptr, gin, false);
 }
 
 void backward(Context& c, Net& n) {
@@ -836,7 +1066,7 @@ void backward(Context& c, Net& n) {
         }
         // head_w and head_b are adjacent in the parameter vector: one ordered sum for both
         LaunchScope ls(c, UWGPU_KERNEL_LEARNED);
-        k_sum_slices<<<nblk(nq, 256), 256, 0, c.stream>>>(nq, (int)hb, n.part.p, n.grads.p + n.head_w);
+        k_sum_slices<<<nblk(nq, 256), 256, 0, c.stream>>>(nq, (int)hb, n.part.p, 0, 0, nullptr, n.grads.p + n.head_w);
     }
     // skip gradients start at zero; the decoder adds into them
     for (int l = 0; l + 1 < L; ++l)
@@ -844,9 +1074,9 @@ void backward(Context& c, Net& n) {
     for (int l = 0; l + 1 < L; ++l) {
         const Vol& g = n.vol[l];
         const int cu = n.ch[l + 1], cs = n.ch[l];
-        relu_bwd(c, g.nv * cs, n.dec_b[l].p, n.g_dec_b[l].p);
+        relu_bwd(c, n, g.nv * cs, n.dec_b[l].p, n.g_dec_b[l].p);
         conv_backward(c, n, g, n.convs[n.dec(l, 1)], n.dec_a[l].p, n.g_dec_b[l].p, n.g_dec_a[l].p);
-        relu_bwd(c, g.nv * cs, n.dec_a[l].p, n.g_dec_a[l].p);
+        relu_bwd(c, n, g.nv * cs, n.dec_a[l].p, n.g_dec_a[l].p);
         conv_backward(c, n, g, n.convs[n.dec(l, 0)], n.dec_cat[l].p, n.g_dec_a[l].p, n.g_cat[l].p);
         float* gcoarse = l + 1 == L - 1 ? n.g_enc_b[L - 1].p : n.g_dec_b[l + 1].p;
         {
@@ -867,9 +1097,9 @@ void backward(Context& c, Net& n) {
             k_pool_bwd_add<<<nblk(g.nv * C, 256), 256, 0, c.stream>>>(g, n.vol[l + 1], C, n.g_in[l + 1].p,
                                                                       n.g_enc_b[l].p);
         }
-        relu_bwd(c, g.nv * C, n.enc_b[l].p, n.g_enc_b[l].p);
+        relu_bwd(c, n, g.nv * C, n.enc_b[l].p, n.g_enc_b[l].p);
         conv_backward(c, n, g, n.convs[n.enc(l, 1)], n.enc_a[l].p, n.g_enc_b[l].p, n.g_enc_a[l].p);
-        relu_bwd(c, g.nv * C, n.enc_a[l].p, n.g_enc_a[l].p);
+        relu_bwd(c, n, g.nv * C, n.enc_a[l].p, n.g_enc_a[l].p);
         const bf16* in = l == 0 ? n.x0.p : n.pool[l - 1].p;
         conv_backward(c, n, g, n.convs[n.enc(l, 0)], in, n.g_enc_a[l].p, n.g_in[l].p);
     }

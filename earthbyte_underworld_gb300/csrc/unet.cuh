@@ -57,6 +57,7 @@ struct Net {
     // gradients (FP32)
     DArray<float> gout, g_enc_a[kMaxLevels], g_enc_b[kMaxLevels], g_in[kMaxLevels];
     DArray<float> g_dec_a[kMaxLevels], g_dec_b[kMaxLevels], g_cat[kMaxLevels];
+    DArray<__nv_bfloat16> g_hi, g_lo;             // BF16 parts of the gradient of the layer being differentiated
     DArray<float> part;                           // per-block partial gradients (ordered sums)
     DArray<uint32_t> tc_err;                      // set by a tensor-core kernel whose MMA wait timed out
 

@@ -1708,9 +1708,14 @@ int gwg_cg32(Context& c, const float* A, const float* dinv, const double* b, flo
 }
 
 // the mixed form's inner solve: G^T W G applied matrix-free from the folded weights Wc
-// (gwg_mf_weights)
+// (gwg_mf_weights); in one launch where the mesh fits the SMs' registers and shared memory
+int gwg_cg_whole(Context& c, const float* Wc, const float* dinv, const double* b, float* x, double rtol, int maxit);   // cg_whole.cu
 int gwg_cg32_mf(Context& c, const float* Wc, const float* dinv, const double* b, float* x, double rtol, int maxit,
                 float* work, double* scal) {
+    if (!c.cc.on) {
+        const int it = gwg_cg_whole(c, Wc, dinv, b, x, rtol, maxit);
+        if (it >= 0) return it;
+    }
     return gwg_cg_T<float>(c, nullptr, Wc, dinv, b, x, rtol, maxit, work, scal);
 }
 

@@ -293,6 +293,7 @@ struct Context {
         DArray<double> einv, s, y, ed;
     } cc;
     std::vector<PcgGraph> pcg_graphs;
+    DArray<uint64_t> cg_words;   // words the blocks of the one-launch inner solve exchange
     cudaEvent_t pcg_events[2] = {nullptr, nullptr};   // the residuals of two queued replays
 
     // learned velocity preconditioner (csrc/unet.cu), created on request

@@ -4,21 +4,22 @@
 // Launched as two kernels per iteration (direction and update), the CG is bound by the launches and by
 // re-reading its vectors from L2: on a 64 x 80 x 112 mesh an iteration moves 27 MB and takes 12 us.  Here
 // the mesh is cut into bricks, one per block and at most one block per SM, and a brick's vectors never
-// leave the block: x, r, p, q and 1/diag of up to eight elements (a piece of a z column) and the weights
-// of up to eleven nodes are in a thread's registers, z with its halo and the weighted gradients at the
-// nodes in shared memory.  Per iteration the blocks exchange only
+// leave the block: r, p and q of up to eight elements (a piece of a z column) and the weights of their
+// nodes are in a thread's registers, x and 1/diag of its elements, z with its halo and the weighted gradients
+// at the nodes in shared memory.  Per iteration the blocks exchange only
 //   - z of the elements on brick faces, as 64-bit words {value, tag}: a reader polls the word until the
 //     tag is the iteration's, so the exchange needs no barrier of its own and no fence;
 //   - the block sums of r.z and p.q, as words of the same kind that every block reads and adds in the same
 //     order.  Each is also the barrier that makes the words of the iteration before free to be overwritten:
 //     a block publishes its p.q only after it has read its halo and every r.z, and its r.z only after every
 //     p.q.
-// An iteration is then bound by the two exchanges (a store, its way through L2 and the load that sees it:
-// 2 to 3 us together with the sums, growing with the blocks that poll) and by the shared-memory reads of the
-// stencil.  Measured per iteration: 64 x 80 x 112 elements 12.3 -> 7.5 us, 64^3 8.3 -> 6.0, 16^3 3.7; a
-// mixed solve on 64 x 80 x 112 (64,200 iterations) 1.24 -> 0.93 s, on 48^3 206 -> 184 ms, on 16^3 29 -> 27 ms.
-// Sixteen copies of the block sums, so that the blocks do not all poll the same lines: 8.2 -> 7.5 us.  Reading
-// the halo only after the sums have come, so that its polling does not disturb theirs, costs 0.5 us more.
+// The sums are exchanged by a warp of their own.  beta does not enter A z, so the other warps read the halo and
+// form A z while that warp waits for r.z; they wait for p.q.  An iteration is then bound by that one wait (a
+// store, its way through L2, the load that sees it and the sums: 1 to 2 us, growing with the blocks that poll),
+// the halo's, and the shared-memory reads of the stencil.  Measured per iteration, two launches -> one warp of
+// sixteen exchanging while the others wait -> this form: 64 x 80 x 112 elements 12.3 -> 7.5 -> 7.1 us, 64^3
+// 8.3 -> 6.0 -> 5.1, 32^3 -> 4.9 -> 3.6, 16^3 -> 3.7 -> 3.2.  Sixteen copies of the block sums, so that the blocks
+// do not all poll the same lines: 8.2 -> 7.5 us on the first mesh.
 //
 // A thread's and a warp's sums are FP32, as in the two-kernel form; above that, where that form adds in
 // FP64, sums are unevaluated pairs of FP32 values (TwoSum, Knuth, The Art of Computer Programming vol. 2,
@@ -36,11 +37,12 @@ namespace uwg {
 
 namespace {
 
-constexpr int kWt = 512;                 // threads of a block
-constexpr int kWWarps = kWt / 32;
+constexpr int kWt = 512;                 // threads that hold elements and nodes
+constexpr int kWWarps = kWt / 32;        // the warp after them exchanges the sums
+constexpr int kWAll = kWt + 32;
 constexpr int kWSeg = 8;                 // elements per thread at most
-constexpr int kWNodes = 11;              // nodes per thread at most
-constexpr int kWHalo = 6;                // halo elements per thread at most, by the threads of all warps but the first
+constexpr int kWRim = 3;                 // nodes of the brick's upper faces per thread at most
+constexpr int kWHalo = 4;                // halo elements per thread at most
 constexpr int kWBlocks = 160;            // blocks at most: five sums per lane
 constexpr int kWCopies = 16;             // copies of the block sums, each read by a sixteenth of the blocks
 static_assert(2 * kWCopies <= 32 && kWWarps == 16, "one lane per word published, each holding the block's sum");
@@ -96,10 +98,10 @@ __device__ __forceinline__ float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-// first warp: publishes the sum of the block's warp sums sw and adds those of all blocks; false when a
+// exchange warp: publishes the sum of the block's warp sums sw and adds those of all blocks; false when a
 // word does not come
 __device__ __forceinline__ bool global_sum(const float* sw, u64* slots, int blocks, uint32_t tag, float& h, float& l) {
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31;
     h = sw[lane % kWWarps];   // the two halves of the warp form the same sum
     l = 0.f;
 #pragma unroll
@@ -144,18 +146,24 @@ __device__ __forceinline__ float pair_ratio(float ah, float al, float bh, float 
     return isfinite(c) ? q + c : q;
 }
 
+// barrier of the whole block, and of the warps that hold elements
+__device__ __forceinline__ void sync_all() { asm volatile("bar.sync 0, %0;" ::"n"(kWAll) : "memory"); }
+__device__ __forceinline__ void sync_work() { asm volatile("bar.sync 1, %0;" ::"n"(kWt) : "memory"); }
+
 template <int SEG>
-__global__ void __launch_bounds__(kWt, 1) k_cg_whole(CgWhole a) {
+__global__ void __launch_bounds__(kWAll, 1) k_cg_whole(CgWhole a) {
     extern __shared__ __align__(16) float smem[];
     __shared__ float sw[kWWarps], sw2[kWWarps];
     __shared__ float s_alpha, s_beta;
     __shared__ int s_stop, s_fail, s_halo;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int zsize = a.nflat + a.hxy + a.hx + 2;
+    const int zsize = a.nflat + (SEG + 1) * a.hxy + a.hx + 2;   // and what short pieces of the last plane read
     float* zb = smem;                                        // z, elements of the brick from (1, 1, 1)
     float* yb = zb + zsize;                                  // [3][node]
-    const int ysize = 3 * a.nflat + SEG * a.hxy + a.hx + 2;  // and what short pieces of the last plane read
-    uint2* list = reinterpret_cast<uint2*>(yb + ysize + ((zsize + ysize) & 1));   // {place in zb, element}
+    const int ysize = 3 * a.nflat + SEG * a.hxy + a.hx + 2;  // likewise
+    float* xs = yb + ysize;                                  // x, [element of the thread][thread]
+    float* ds = xs + SEG * kWt;                              // 1/diag, the same
+    uint2* list = reinterpret_cast<uint2*>(ds + SEG * kWt + ((zsize + ysize) & 1));   // {place in zb, element}
     const int ix = blockIdx.x % a.nbx, iy = blockIdx.x / a.nbx % a.nby, iz = blockIdx.x / (a.nbx * a.nby);
     const int x0 = ix * a.bx, y0 = iy * a.by, z0 = iz * a.bz;
     const int cx = min(a.bx, a.ex - x0), cy = min(a.by, a.ey - y0), cz = min(a.bz, a.ez - z0);   // this brick
@@ -164,10 +172,10 @@ __global__ void __launch_bounds__(kWt, 1) k_cg_whole(CgWhole a) {
         s_fail = 0;
         s_halo = 0;
     }
-    for (int i = tid; i < zsize; i += kWt) zb[i] = 0.f;
+    for (int i = tid; i < zsize; i += kWAll) zb[i] = 0.f;
     __syncthreads();
     // halo elements inside the mesh (the others stay zero)
-    for (int i = tid; i < (cz + 2) * (cy + 2) * (cx + 2); i += kWt) {
+    for (int i = tid; i < (cz + 2) * (cy + 2) * (cx + 2); i += kWAll) {
         const int hx = i % (cx + 2), t = i / (cx + 2), hy = t % (cy + 2), hz = t / (cy + 2);
         const bool inner = hx >= 1 && hx <= cx && hy >= 1 && hy <= cy && hz >= 1 && hz <= cz;
         const int gx = x0 + hx - 1, gy = y0 + hy - 1, gz = z0 + hz - 1;
@@ -175,68 +183,19 @@ __global__ void __launch_bounds__(kWt, 1) k_cg_whole(CgWhole a) {
             list[atomicAdd(&s_halo, 1)] = make_uint2((unsigned)(hx + a.hx * hy + a.hxy * hz),
                                                      (unsigned)(gx + a.ex * (gy + a.ey * gz)));
     }
-    // this thread's elements: `cnt` of the column (tx, ty) from plane tz
-    const int cols = a.bx * a.by, col = tid % cols, tx = col % a.bx, ty = col / a.bx, tz = tid / cols * a.seg;
-    const int cnt = tx < cx && ty < cy ? max(0, min(a.seg, cz - tz)) : 0;
-    const int e0 = (x0 + tx) + a.ex * ((y0 + ty) + a.ey * (z0 + tz)), exy = a.ex * a.ey;
-    const int n0 = cnt > 0 ? tx + a.hx * ty + a.hxy * tz : 0;   // lower corner node of the first
-    const int c0 = n0 + 1 + a.hx + a.hxy;
-    float x[SEG], r[SEG], p[SEG], q[SEG], d[SEG];
-    unsigned faces = 0;
-#pragma unroll
-    for (int j = 0; j < SEG; ++j) {
-        const bool in = j < cnt;
-        r[j] = in ? (float)a.b[e0 + j * exy] : 0.f;
-        d[j] = in ? a.dinv[e0 + j * exy] : 0.f;
-        x[j] = p[j] = q[j] = 0.f;
-        if (in && (tx == 0 || tx == cx - 1 || ty == 0 || ty == cy - 1 || tz + j == 0 || tz + j == cz - 1)) faces |= 1u << j;
-    }
-    float w[kWNodes][3];
-#pragma unroll
-    for (int m = 0; m < kWNodes; ++m) {
-        const int n = tid + m * kWt, nx = n % a.hx, ny = n / a.hx % (a.hxy / a.hx), nz = n / a.hxy;
-        const bool in = n < a.nflat && nx <= cx && ny <= cy && nz <= cz;
-        const int64_t o = in ? (x0 + nx) + a.pitch * ((y0 + ny) + a.nny * (int64_t)(z0 + nz)) : 0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) w[m][k] = in ? __ldg(a.Wc + k * a.nn + o) : 0.f;
-    }
-    __syncthreads();
-    const int nh = s_halo, blocks = gridDim.x;
     u64* rz_slots = a.sums;
     u64* pq_slots = rz_slots + 2 * kWBlocks * kWCopies;
     u64* rr_slots = pq_slots + 2 * kWBlocks * kWCopies;
-    float rz_h = 0.f, rz_l = 0.f, pq_h = 0.f, pq_l = 0.f;    // first warp: r.z and p.q of the last sums
-    double norm0 = 0.0;                                      // first warp
-    int code = 0, k = -1;
+    const int blocks = gridDim.x;
     // k = -1: z = 1/diag b, p = z, q = A z; then iteration k: x, r, z with alpha, r.z, p and q with beta, p.q
-    for (;; ++k) {
-        const uint32_t tag = (uint32_t)(k + 2);
-        const bool check = k < 0 || (k + 1) % kWCheck == 0;
-        {
-            const float alpha = k < 0 ? 0.f : s_alpha;
-            float rz = 0.f, rr = 0.f;
-#pragma unroll
-            for (int j = 0; j < SEG; ++j)
-                if (j < cnt) {
-                    if (k >= 0) {
-                        x[j] = fmaf(alpha, p[j], x[j]);
-                        r[j] = fmaf(-alpha, q[j], r[j]);
-                    }
-                    const float z = r[j] * d[j];
-                    zb[c0 + j * a.hxy] = z;
-                    if (faces >> j & 1u) st_word(a.face + e0 + j * exy, z, tag);
-                    rz = fmaf(r[j], z, rz);
-                    rr = fmaf(r[j], r[j], rr);
-                }
-            rz = warp_sum(rz);
-            if (check) rr = warp_sum(rr);
-            if (lane == 0) {
-                sw[warp] = rz;
-                sw2[warp] = rr;
-            }
-        }
-        __syncthreads();
-        if (warp == 0) {
+    if (warp == kWWarps) {
+        float rz_h = 0.f, rz_l = 0.f, pq_h, pq_l;   // r.z and p.q of the last sums
+        double norm0 = 0.0;
+        sync_all();
+        for (int k = -1;; ++k) {
+            const uint32_t tag = (uint32_t)(k + 2);
+            const bool check = k < 0 || (k + 1) % kWCheck == 0;
+            sync_all();
             float h, l, h2 = 0.f, l2 = 0.f;
             bool ok = global_sum(sw, rz_slots, blocks, tag, h, l);
             if (check) ok = global_sum(sw2, rr_slots, blocks, tag, h2, l2) && ok;
@@ -246,9 +205,9 @@ __global__ void __launch_bounds__(kWt, 1) k_cg_whole(CgWhole a) {
                 if (check) {
                     const double norm = sqrt((double)h2 + (double)l2);
                     if (k < 0) norm0 = norm;
-                    code = !(norm0 > 0.0) ? 1 : !isfinite(norm) ? 2 : k >= 0 && norm <= a.rtol * norm0 ? 3
-                         : k + 1 >= a.maxit ? 4 : 0;
-                    s_stop = code != 0;
+                    const int code = !(norm0 > 0.0) ? 1 : !isfinite(norm) ? 2 : k >= 0 && norm <= a.rtol * norm0 ? 3
+                                   : k + 1 >= a.maxit ? 4 : 0;
+                    s_stop = code;
                     if (code && blockIdx.x == 0) {
                         a.report[0] = k + 1;
                         a.report[1] = code;
@@ -259,15 +218,103 @@ __global__ void __launch_bounds__(kWt, 1) k_cg_whole(CgWhole a) {
             }
             rz_h = h;
             rz_l = l;
+            sync_all();
+            if (s_fail || s_stop) break;
+            sync_all();
+            ok = global_sum(sw, pq_slots, blocks, tag, pq_h, pq_l);
+            if (lane == 0) {
+                s_alpha = pair_ratio(rz_h, rz_l, pq_h, pq_l);
+                if (!ok) s_fail = 1;
+            }
+            sync_all();
+            if (s_fail) break;
+        }
+        if (s_fail && lane == 0) atomicExch(a.failed, 1);
+        return;
+    }
+    // this thread's elements: `cnt` of the column (tx, ty) from plane tz
+    const int cols = a.bx * a.by, col = tid % cols, tx = col % a.bx, ty = col / a.bx, tz = tid / cols * a.seg;
+    const int cnt = tx < cx && ty < cy ? max(0, min(a.seg, cz - tz)) : 0;
+    const int e0 = (x0 + tx) + a.ex * ((y0 + ty) + a.ey * (z0 + tz)), exy = a.ex * a.ey;
+    const int n0 = cnt > 0 ? tx + a.hx * ty + a.hxy * tz : 0;   // lower corner node of the first
+    const int c0 = n0 + 1 + a.hx + a.hxy;
+    float r[SEG], p[SEG], q[SEG];
+    unsigned faces = 0;
+#pragma unroll
+    for (int j = 0; j < SEG; ++j) {
+        const bool in = j < cnt;
+        r[j] = in ? (float)a.b[e0 + j * exy] : 0.f;
+        ds[j * kWt + tid] = in ? a.dinv[e0 + j * exy] : 0.f;
+        p[j] = q[j] = 0.f;
+        xs[j * kWt + tid] = 0.f;
+        if (in && (tx == 0 || tx == cx - 1 || ty == 0 || ty == cy - 1 || tz + j == 0 || tz + j == cz - 1)) faces |= 1u << j;
+    }
+    // weights of its nodes: the lower corner node of each of its elements, and some nodes on the upper faces
+    // of the brick (x = cx, then y = cy, then z = cz)
+    auto weight = [&](int nx, int ny, int nz, bool in, float* to) {
+        const int64_t o = in ? (x0 + nx) + a.pitch * ((y0 + ny) + a.nny * (int64_t)(z0 + nz)) : 0;
+        for (int k = 0; k < 3; ++k) to[k] = in ? __ldg(a.Wc + k * a.nn + o) : 0.f;
+    };
+    float w[SEG][3], wr[kWRim][3];
+    int rim[kWRim];
+#pragma unroll
+    for (int j = 0; j < SEG; ++j) weight(tx, ty, tz + j, j < cnt, w[j]);
+    const int fx = (cy + 1) * (cz + 1), fy = cx * (cz + 1), fz = cx * cy;
+#pragma unroll
+    for (int m = 0; m < kWRim; ++m) {
+        int i = tid + m * kWt, nx, ny, nz;
+        const bool in = i < fx + fy + fz;
+        if (i < fx) {
+            nx = cx;
+            ny = i % (cy + 1);
+            nz = i / (cy + 1);
+        } else if ((i -= fx) < fy) {
+            nx = i % cx;
+            ny = cy;
+            nz = i / cx;
         } else {
-            const int first = tid - 32;
+            i -= fy;
+            nx = i % cx;
+            ny = i / cx;
+            nz = cz;
+        }
+        rim[m] = in ? nx + a.hx * ny + a.hxy * nz : -1;
+        weight(nx, ny, nz, in, wr[m]);
+    }
+    sync_all();
+    const int nh = s_halo;
+    for (int k = -1;; ++k) {
+        const uint32_t tag = (uint32_t)(k + 2);
+        {
+            const float alpha = k < 0 ? 0.f : s_alpha;
+            float rz = 0.f, rr = 0.f;
+#pragma unroll
+            for (int j = 0; j < SEG; ++j)
+                if (j < cnt) {
+                    if (k >= 0) {
+                        xs[j * kWt + tid] = fmaf(alpha, p[j], xs[j * kWt + tid]);
+                        r[j] = fmaf(-alpha, q[j], r[j]);
+                    }
+                    const float z = r[j] * ds[j * kWt + tid];
+                    zb[c0 + j * a.hxy] = z;
+                    if (faces >> j & 1u) st_word(a.face + e0 + j * exy, z, tag);
+                    rz = fmaf(r[j], z, rz);
+                    rr = fmaf(r[j], r[j], rr);
+                }
+            rz = warp_sum(rz);
+            if (k < 0 || (k + 1) % kWCheck == 0) rr = warp_sum(rr);
+            if (lane == 0) {
+                sw[warp] = rz;
+                sw2[warp] = rr;
+            }
+        }
+        sync_all();
+        // while the exchange warp waits for r.z: the halo, and A z, which beta does not enter
+        {
             u64 v[kWHalo];
             uint2 at[kWHalo];
 #pragma unroll
-            for (int m = 0; m < kWHalo; ++m) {
-                const int i = first + m * (kWt - 32);
-                at[m] = i < nh ? list[i] : make_uint2(0xffffffffu, 0u);
-            }
+            for (int m = 0; m < kWHalo; ++m) at[m] = tid + m * kWt < nh ? list[tid + m * kWt] : make_uint2(0xffffffffu, 0u);
             bool all = false;
             for (int tries = 0; tries < kWPoll && !all; ++tries) {
                 all = true;
@@ -283,67 +330,81 @@ __global__ void __launch_bounds__(kWt, 1) k_cg_whole(CgWhole a) {
                 if (at[m].x != 0xffffffffu) zb[at[m].x] = word_value(v[m]);
             if (!all) s_fail = 1;
         }
-        __syncthreads();
-        if (s_fail || s_stop) break;
-        // nodes: y_d = W_d (sum of z above the node along d - sum below)
+        sync_work();
+        // nodes: y_d = W_d (sum of z above the node along d - sum below).  A thread's own nodes lie above one
+        // another and share the sums of an element plane: 4 + 3 shared-memory accesses each instead of 8 + 3
+        {
+            float gx = 0.f, gy = 0.f, z00 = 0.f, z10 = 0.f, z01 = 0.f, z11 = 0.f;
 #pragma unroll
-        for (int m = 0; m < kWNodes; ++m) {
-            const int n = tid + m * kWt;
-            if (n < a.nflat) {
-                const float* f = zb + n;
+            for (int j = 0; j <= SEG; ++j) {   // of a short piece the planes above it are read and not used
+                const float* f = zb + n0 + j * a.hxy;
+                const float f00 = f[0], f10 = f[1], f01 = f[a.hx], f11 = f[a.hx + 1];
+                const float hx = (f10 - f00) + (f11 - f01), hy = (f01 - f00) + (f11 - f10);
+                if (j > 0 && j <= cnt) {
+                    float* y = yb + n0 + (j - 1) * a.hxy;
+                    y[0] = w[j - 1][0] * (gx + hx);
+                    y[a.nflat] = w[j - 1][1] * (gy + hy);
+                    y[2 * a.nflat] = w[j - 1][2] * (((f00 - z00) + (f10 - z10)) + ((f01 - z01) + (f11 - z11)));
+                }
+                gx = hx;
+                gy = hy;
+                z00 = f00;
+                z10 = f10;
+                z01 = f01;
+                z11 = f11;
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < kWRim; ++m)
+            if (rim[m] >= 0) {
+                const float* f = zb + rim[m];
                 const float* g = f + a.hxy;
+                float* y = yb + rim[m];
                 const float z000 = f[0], z100 = f[1], z010 = f[a.hx], z110 = f[a.hx + 1];
                 const float z001 = g[0], z101 = g[1], z011 = g[a.hx], z111 = g[a.hx + 1];
-                yb[n] = w[m][0] * (((z100 - z000) + (z110 - z010)) + ((z101 - z001) + (z111 - z011)));
-                yb[a.nflat + n] = w[m][1] * (((z010 - z000) + (z110 - z100)) + ((z011 - z001) + (z111 - z101)));
-                yb[2 * a.nflat + n] = w[m][2] * (((z001 - z000) + (z101 - z100)) + ((z011 - z010) + (z111 - z110)));
+                y[0] = wr[m][0] * (((z100 - z000) + (z110 - z010)) + ((z101 - z001) + (z111 - z011)));
+                y[a.nflat] = wr[m][1] * (((z010 - z000) + (z110 - z100)) + ((z011 - z001) + (z111 - z101)));
+                y[2 * a.nflat] = wr[m][2] * (((z001 - z000) + (z101 - z100)) + ((z011 - z010) + (z111 - z110)));
+            }
+        sync_work();
+        // elements: A z from the two node planes of each, the lower one kept from the element below
+        float az[SEG];
+        {
+            float lo_xy = 0.f, lo_z = 0.f;
+#pragma unroll
+            for (int j = 0; j <= SEG; ++j) {   // planes above a short piece are read and not used
+                const float* y = yb + n0 + j * a.hxy;
+                const float* y1 = y + a.nflat;
+                const float* y2 = y1 + a.nflat;
+                const float gx = (y[0] - y[1]) + (y[a.hx] - y[a.hx + 1]);
+                const float gy = (y1[0] - y1[a.hx]) + (y1[1] - y1[a.hx + 1]);
+                const float gz = (y2[0] + y2[1]) + (y2[a.hx] + y2[a.hx + 1]);
+                if (j > 0) az[j - 1] = (lo_xy + (gx + gy)) + (lo_z - gz);
+                lo_xy = gx + gy;
+                lo_z = gz;
             }
         }
-        __syncthreads();
-        // elements: A z from the two node planes of each, the lower one kept from the element below
+        sync_all();
+        if (s_fail || s_stop) break;
         const float beta = s_beta;
         float pq = 0.f;
-        float lo_xy = 0.f, lo_z = 0.f;
 #pragma unroll
-        for (int j = 0; j <= SEG; ++j) {   // planes above a short piece are read and not used
-            const float* y = yb + n0 + j * a.hxy;
-            const float* y1 = y + a.nflat;
-            const float* y2 = y1 + a.nflat;
-            const float gx = (y[0] - y[1]) + (y[a.hx] - y[a.hx + 1]);
-            const float gy = (y1[0] - y1[a.hx]) + (y1[1] - y1[a.hx + 1]);
-            const float gz = (y2[0] + y2[1]) + (y2[a.hx] + y2[a.hx + 1]);
-            if (j > 0) {
-                const float az = (lo_xy + (gx + gy)) + (lo_z - gz);
-                const float z = zb[c0 + (j - 1) * a.hxy];
-                if (j <= cnt) {
-                    p[j - 1] = fmaf(beta, p[j - 1], z);
-                    q[j - 1] = fmaf(beta, q[j - 1], az);
-                    pq = fmaf(p[j - 1], q[j - 1], pq);
-                }
+        for (int j = 0; j < SEG; ++j)
+            if (j < cnt) {
+                p[j] = fmaf(beta, p[j], zb[c0 + j * a.hxy]);
+                q[j] = fmaf(beta, q[j], az[j]);
+                pq = fmaf(p[j], q[j], pq);
             }
-            lo_xy = gx + gy;
-            lo_z = gz;
-        }
         pq = warp_sum(pq);
         if (lane == 0) sw[warp] = pq;
-        __syncthreads();
-        if (warp == 0) {
-            const bool ok = global_sum(sw, pq_slots, blocks, tag, pq_h, pq_l);
-            if (lane == 0) {
-                s_alpha = pair_ratio(rz_h, rz_l, pq_h, pq_l);
-                if (!ok) s_fail = 1;
-            }
-        }
-        __syncthreads();
+        sync_all();
+        sync_all();
         if (s_fail) break;
     }
-    if (s_fail) {
-        if (tid == 0) atomicExch(a.failed, 1);
-        return;
-    }
+    if (s_fail) return;
 #pragma unroll
     for (int j = 0; j < SEG; ++j)
-        if (j < cnt) a.x[e0 + j * exy] = x[j];
+        if (j < cnt) a.x[e0 + j * exy] = xs[j * kWt + tid];
 }
 
 // the instance of the kernel: elements per thread, rounded up to a power of two
@@ -359,7 +420,7 @@ const void* kernel_of(const CgWhole& a) {
 
 // Cuts the mesh into bricks for `sms` blocks at most.  Among the cuts whose brick fits a block (elements,
 // nodes and halo per thread as above) the one with the least work per thread, weighed by instructions:
-// 40 per node, 45 per element, 30 per halo element.  False when no cut fits.
+// 40 per node of the upper faces, 70 per element with its lower corner node, 30 per halo element.  False when no cut fits.
 bool cut(CgWhole& a, int sms, size_t* smem) {
     double best = 1e300;
     if (sms > kWBlocks) sms = kWBlocks;
@@ -375,9 +436,10 @@ bool cut(CgWhole& a, int sms, size_t* smem) {
                 const int pieces = kWt / (bx * by), seg = (bz + pieces - 1) / pieces;
                 const int nflat = (bz + 1) * (by + 2) * (bx + 2);
                 const int halo = (bx + 2) * (by + 2) * (bz + 2) - bx * by * bz;
-                if (seg > kWSeg || nflat > kWNodes * kWt || halo > kWHalo * (kWt - 32)) continue;
-                const double cost = 40.0 * ((nflat + kWt - 1) / kWt) + 45.0 * (seg + 1) * (bx % 32 ? 1.2 : 1.0) +
-                                    30.0 * ((halo + kWt - 33) / (kWt - 32)) + 0.01 * nx * ny * nz;
+                const int rim = (bx + 1) * (by + 1) * (bz + 1) - bx * by * bz;
+                if (seg > kWSeg || rim > kWRim * kWt || halo > kWHalo * kWt) continue;
+                const double cost = 40.0 * ((rim + kWt - 1) / kWt) + 70.0 * (seg + 1) * (bx % 32 ? 1.2 : 1.0) +
+                                    30.0 * ((halo + kWt - 1) / kWt) + 0.01 * nx * ny * nz;
                 if (cost < best) {
                     best = cost;
                     a.bx = bx;
@@ -396,8 +458,8 @@ bool cut(CgWhole& a, int sms, size_t* smem) {
         }
     }
     if (best == 1e300) return false;
-    *smem = sizeof(float) * ((size_t)a.nflat + a.hxy + a.hx + 2 + 3 * (size_t)a.nflat +
-                              (size_t)(seg_of(a) + 1) * a.hxy + a.hx + 3) +
+    const size_t n = seg_of(a);
+    *smem = sizeof(float) * (4 * (size_t)a.nflat + (2 * n + 1) * a.hxy + 2 * (size_t)a.hx + 5 + 2 * n * kWt) +
             sizeof(uint2) * a.halo;
     return true;
 }
@@ -441,7 +503,7 @@ int gwg_cg_whole(Context& c, const float* Wc, const float* dinv, const double* b
     {
         LaunchScope ls(c, UWGPU_KERNEL_SCHUR_PC);
         void* args[] = {(void*)&a};
-        UWG_CUDA(cudaLaunchCooperativeKernel(kernel_of(a), dim3((unsigned)(a.nbx * a.nby * a.nbz)), dim3(kWt),
+        UWG_CUDA(cudaLaunchCooperativeKernel(kernel_of(a), dim3((unsigned)(a.nbx * a.nby * a.nbz)), dim3(kWAll),
                                              args, smem, c.stream));
     }
     double* h = c.host_scalars;

@@ -154,9 +154,22 @@ __global__ void k_convert(int64_t n, const S* __restrict__ a, D* __restrict__ b)
 // row w % DIM of 32 consecutive nodes (lanes), so every stencil load of a warp is coalesced and a
 // node's DIM rows run on DIM threads (three times the parallelism of one thread per node).
 constexpr int kRowThreads = 192;
+// Blocks per SM asked of the compiler for the kernels that stream a stencil (bound by the bytes in flight): left
+// alone it fits 32 registers and ten blocks and issues a row's loads a few at a time.  Five to seven were tried;
+// with six and the streaming loads below, on the 65 x 81 x 113 nodes of a mixed solve's fine level: Chebyshev step
+// 86 -> 69 us (5.3 TB/s), residual 100 -> 62, FP32 apply 120 -> 100 (5.9 TB/s), FP64 apply 272 -> 242 (FP64-bound).
+constexpr int kRowBlocks = 6;
+
+// Stencil entry: read once per kernel.  STREAM (a stencil larger than L2): marked to leave the caches first,
+// where it would push out the vectors, which are read 27 times (FP32 apply 104 -> 100 us, Chebyshev step 80 -> 69).
+// A stencil that L2 holds is read the ordinary way: the next sweep finds it there (8 -> 10 us otherwise).
+template <bool STREAM, typename T>
+__device__ __forceinline__ T ld_entry(const T* p) {
+    return STREAM ? __ldcs(p) : __ldg(p);
+}
 
 // sum_q sum_c A[q][r][c][n] x[c][m(q)] for one row r of node n
-template <int DIM, typename T>
+template <int DIM, typename T, bool STREAM = false>
 __device__ __forceinline__ T stencil_row_r(const Grid& g, int64_t n, int64_t i, int64_t j, int64_t k, int r,
                                            const T* __restrict__ A, const T* __restrict__ x) {
     constexpr int NB = nblocks<DIM>();
@@ -175,7 +188,7 @@ __device__ __forceinline__ T stencil_row_r(const Grid& g, int64_t n, int64_t i, 
             const int64_t m = n + o.dx[q % 3] + o.dy[(q / 3) % 3] + o.dz[DIM == 3 ? q / 9 : 1];
 #pragma unroll
             for (int cc = 0; cc < DIM; ++cc) {
-                a[qq * DIM + cc] = __ldg(A + ((int64_t)(q * DIM + r) * DIM + cc) * g.nn + n);
+                a[qq * DIM + cc] = ld_entry<STREAM>(A + ((int64_t)(q * DIM + r) * DIM + cc) * g.nn + n);
                 xv[qq * DIM + cc] = x[(int64_t)cc * g.nn + m];
             }
         }
@@ -189,7 +202,7 @@ __device__ __forceinline__ T stencil_row_r(const Grid& g, int64_t n, int64_t i, 
 // multiplies by S16[r][n].  The FP16 entries of neighbours q = 2p and 2p + 1 share one 32-bit word,
 // [p][r][c][node], so a load brings two entries and one conversion widens both.  Loads go out in
 // batches of five pairs.
-template <int DIM>
+template <int DIM, bool STREAM>
 __device__ __forceinline__ float stencil_row_h(const Grid& g, int64_t n, int64_t i, int64_t j, int64_t k, int r,
                                                const uint32_t* __restrict__ A, const float* __restrict__ x) {
     constexpr int NB = nblocks<DIM>(), NP = (NB + 1) / 2, PB = 5;
@@ -208,7 +221,7 @@ __device__ __forceinline__ float stencil_row_h(const Grid& g, int64_t n, int64_t
                 const int64_t m1 = q1 < NB ? n + o.dx[q1 % 3] + o.dy[(q1 / 3) % 3] + o.dz[DIM == 3 ? q1 / 9 : 1] : n;
 #pragma unroll
                 for (int cc = 0; cc < DIM; ++cc) {
-                    w[pp * DIM + cc] = __ldg(A + ((int64_t)(pr * DIM + r) * DIM + cc) * g.nn + n);
+                    w[pp * DIM + cc] = ld_entry<STREAM>(A + ((int64_t)(pr * DIM + r) * DIM + cc) * g.nn + n);
                     xv[(2 * pp) * DIM + cc] = x[(int64_t)cc * g.nn + m0];
                     xv[(2 * pp + 1) * DIM + cc] = q1 < NB ? x[(int64_t)cc * g.nn + m1] : 0.f;
                 }
@@ -231,8 +244,8 @@ __device__ __forceinline__ float stencil_row_h(const Grid& g, int64_t n, int64_t
 }
 
 // r = b - A x with the FP16 stencil (V-cycle residuals of the mixed form)
-template <int DIM>
-__global__ void __launch_bounds__(kRowThreads) k_residual_h(Grid g, const uint32_t* __restrict__ A,
+template <int DIM, bool STREAM>
+__global__ void __launch_bounds__(kRowThreads, kRowBlocks) k_residual_h(Grid g, const uint32_t* __restrict__ A,
                                                             const float* __restrict__ S, const float* __restrict__ x,
                                                             const float* __restrict__ b, float* __restrict__ y) {
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -242,7 +255,7 @@ __global__ void __launch_bounds__(kRowThreads) k_residual_h(Grid g, const uint32
     int64_t i, j, k;
     node_ijk<DIM>(g, n, i, j, k);
     const int64_t idx = (int64_t)r * g.nn + n;
-    y[idx] = b[idx] - S[idx] * stencil_row_h<DIM>(g, n, i, j, k, r, A, x);
+    y[idx] = b[idx] - S[idx] * stencil_row_h<DIM, STREAM>(g, n, i, j, k, r, A, x);
 }
 
 // FP32 -> FP16 row-scaled stencil: S16[r][n] = max over the row's entries of |A|; the entries of
@@ -272,8 +285,8 @@ __global__ void k_to_fp16_rows(Grid g, const float* __restrict__ A, uint32_t* __
 }
 
 // y = A x (or r = b - A x when b is given), row-split
-template <int DIM, typename T>
-__global__ void __launch_bounds__(kRowThreads) k_apply(Grid g, const T* __restrict__ A, const T* __restrict__ x,
+template <int DIM, typename T, bool STREAM>
+__global__ void __launch_bounds__(kRowThreads, kRowBlocks) k_apply(Grid g, const T* __restrict__ A, const T* __restrict__ x,
                                                        const T* __restrict__ b, T* __restrict__ y) {
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int r = warp % DIM, grp = warp / DIM;
@@ -281,7 +294,7 @@ __global__ void __launch_bounds__(kRowThreads) k_apply(Grid g, const T* __restri
     if (n >= g.nn) return;
     int64_t i, j, k;
     node_ijk<DIM>(g, n, i, j, k);
-    T v = stencil_row_r<DIM, T>(g, n, i, j, k, r, A, x);
+    T v = stencil_row_r<DIM, T, STREAM>(g, n, i, j, k, r, A, x);
     y[(int64_t)r * g.nn + n] = b ? b[(int64_t)r * g.nn + n] - v : v;
 }
 
@@ -341,8 +354,8 @@ __global__ void __launch_bounds__(kRowThreads) k_cheb_step(Grid g, const T* __re
 }
 
 // The Chebyshev step with the FP16 row-scaled stencil (mixed form)
-template <int DIM>
-__global__ void __launch_bounds__(kRowThreads) k_cheb_step_h(Grid g, const uint32_t* __restrict__ A,
+template <int DIM, bool STREAM>
+__global__ void __launch_bounds__(kRowThreads, kRowBlocks) k_cheb_step_h(Grid g, const uint32_t* __restrict__ A,
                                                              const float* __restrict__ S, const float* __restrict__ Dinv,
                                                              const float* __restrict__ b, const float* __restrict__ xin,
                                                              float* __restrict__ xout, float* __restrict__ d, float c1,
@@ -358,7 +371,7 @@ __global__ void __launch_bounds__(kRowThreads) k_cheb_step_h(Grid g, const uint3
         node_ijk<DIM>(g, n, i, j, k);
         const int64_t idx = (int64_t)r * g.nn + n;
         res = b[idx];
-        if (xin) res -= S[idx] * stencil_row_h<DIM>(g, n, i, j, k, r, A, xin);
+        if (xin) res -= S[idx] * stencil_row_h<DIM, STREAM>(g, n, i, j, k, r, A, xin);
     }
     sres[threadIdx.x] = res;
     __syncthreads();
@@ -900,16 +913,34 @@ const double* dinv_of<double>(const Level& L) { return L.Dinv64.p; }
 template <>
 const float* dinv_of<float>(const Level& L) { return L.Dinv32.p; }
 
+// whether a stencil of `bytes` is larger than L2
+static bool streams(Context& c, double bytes) {
+    int l2 = 0;
+    UWG_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c.device));
+    return bytes > (double)l2;
+}
+
+static bool streams16(Context& c, const Grid& g) { return g.dim == 3 && streams(c, (double)g.nn * 14 * 9 * 4); }
+
+// y = A x, or b - A x when b is given
+template <typename T>
+static void launch_apply(Context& c, const Grid& g, const Level& L, const T* x, const T* b, T* y) {
+    const T* A = stencil_of<T>(L);
+    if (g.dim == 2)
+        k_apply<2, T, false><<<blocks_for(g.nn, kRowThreads / 2), kRowThreads, 0, c.stream>>>(g, A, x, b, y);
+    else if (streams(c, (double)g.nn * 243 * sizeof(T)))
+        k_apply<3, T, true><<<blocks_for(g.nn, kRowThreads / 3), kRowThreads, 0, c.stream>>>(g, A, x, b, y);
+    else
+        k_apply<3, T, false><<<blocks_for(g.nn, kRowThreads / 3), kRowThreads, 0, c.stream>>>(g, A, x, b, y);
+}
+
 template <typename T>
 void level_apply(Context& c, const Level& L, const T* x, T* y) {
     Grid g = grid_of(L.mesh);
     int D = g.dim, NB = D == 3 ? 27 : 9;
     note_work(c, UWGPU_KERNEL_APPLY, (double)g.nn * (NB * D * D + 2 * D) * sizeof(T), 2.0 * g.nn * NB * D * D);
     LaunchScope ls(c, UWGPU_KERNEL_APPLY);
-    if (g.dim == 3)
-        k_apply<3, T><<<blocks_for(g.nn, kRowThreads / 3), kRowThreads, 0, c.stream>>>(g, stencil_of<T>(L), x, nullptr, y);
-    else
-        k_apply<2, T><<<blocks_for(g.nn, kRowThreads / 2), kRowThreads, 0, c.stream>>>(g, stencil_of<T>(L), x, nullptr, y);
+    launch_apply<T>(c, g, L, x, nullptr, y);
 }
 
 template <typename T>
@@ -920,19 +951,14 @@ void level_residual(Context& c, const Level& L, const T* x, const T* b, T* r) {
         if (L.has16 && c.smooth16) {
             note_work(c, UWGPU_KERNEL_APPLY, (double)g.nn * ((NB + 1) / 2 * D * D * 4 + 4 * D * 4), 2.0 * g.nn * NB * D * D);
             LaunchScope ls(c, UWGPU_KERNEL_APPLY);
-            if (g.dim == 3)
-                k_residual_h<3><<<blocks_for(g.nn, kRowThreads / 3), kRowThreads, 0, c.stream>>>(g, L.A16.p, L.S16.p, x, b, r);
-            else
-                k_residual_h<2><<<blocks_for(g.nn, kRowThreads / 2), kRowThreads, 0, c.stream>>>(g, L.A16.p, L.S16.p, x, b, r);
+            auto kern = g.dim == 2 ? k_residual_h<2, false> : streams16(c, g) ? k_residual_h<3, true> : k_residual_h<3, false>;
+            kern<<<blocks_for(g.nn, kRowThreads / g.dim), kRowThreads, 0, c.stream>>>(g, L.A16.p, L.S16.p, x, b, r);
             return;
         }
     }
     note_work(c, UWGPU_KERNEL_APPLY, (double)g.nn * (NB * D * D + 3 * D) * sizeof(T), 2.0 * g.nn * NB * D * D);
     LaunchScope ls(c, UWGPU_KERNEL_APPLY);
-    if (g.dim == 3)
-        k_apply<3, T><<<blocks_for(g.nn, kRowThreads / 3), kRowThreads, 0, c.stream>>>(g, stencil_of<T>(L), x, b, r);
-    else
-        k_apply<2, T><<<blocks_for(g.nn, kRowThreads / 2), kRowThreads, 0, c.stream>>>(g, stencil_of<T>(L), x, b, r);
+    launch_apply<T>(c, g, L, x, b, r);
 }
 
 // symmetric sweep: colours ascending then descending
@@ -1050,12 +1076,9 @@ void level_cheb(Context& c, Level& L, const T* b, T* x, int degree, bool zero_in
         LaunchScope ls(c, UWGPU_KERNEL_SMOOTH);
         if constexpr (std::is_same<T, float>::value) {
             if (half) {
-                if (D == 3)
-                    k_cheb_step_h<3><<<blocks_for(g.nn, kRowThreads / 3), kRowThreads, 0, c.stream>>>(
-                        g, L.A16.p, L.S16.p, L.Dinv32.p, b, cur, dst, d, (float)c1, (float)c2, k == 0);
-                else
-                    k_cheb_step_h<2><<<blocks_for(g.nn, kRowThreads / 2), kRowThreads, 0, c.stream>>>(
-                        g, L.A16.p, L.S16.p, L.Dinv32.p, b, cur, dst, d, (float)c1, (float)c2, k == 0);
+                auto kern = D == 2 ? k_cheb_step_h<2, false> : streams16(c, g) ? k_cheb_step_h<3, true> : k_cheb_step_h<3, false>;
+                kern<<<blocks_for(g.nn, kRowThreads / D), kRowThreads, 0, c.stream>>>(
+                    g, L.A16.p, L.S16.p, L.Dinv32.p, b, cur, dst, d, (float)c1, (float)c2, k == 0);
                 cur = dst;
                 continue;
             }

@@ -466,22 +466,36 @@ bool cut(CgWhole& a, int sms, size_t* smem) {
 
 }  // namespace
 
-// Solves G^T W G x = b as gwg_cg32_mf describes.  Returns the iterations taken, or -1 when the mesh has no
-// cut into bricks that fit (more than about 600,000 elements on 152 SMs).
-int gwg_cg_whole(Context& c, const float* Wc, const float* dinv, const double* b, float* x, double rtol, int maxit) {
+namespace {
+bool plan(Context& c, CgWhole& a, size_t* smem) {
     const MeshDesc& m = c.levels[0].mesh;
-    if (m.dim != 3 || m.ne >= ((int64_t)1 << 31)) return -1;
+    if (m.dim != 3 || m.ne >= ((int64_t)1 << 31)) return false;
     int sms = 0, coop = 0, optin = 0;
     UWG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
     UWG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c.device));
     UWG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device));
-    if (!coop) return -1;
-    CgWhole a{};
+    if (!coop) return false;
     a.ex = (int)m.nel[0];
     a.ey = (int)m.nel[1];
     a.ez = (int)m.nel[2];
+    return cut(a, sms, smem) && *smem + 1024 <= (size_t)optin;
+}
+}  // namespace
+
+// whether gwg_cg_whole solves on the context's mesh
+bool gwg_cg_whole_fits(Context& c) {
+    CgWhole a{};
     size_t smem = 0;
-    if (!cut(a, sms, &smem) || smem + 1024 > (size_t)optin) return -1;
+    return plan(c, a, &smem);
+}
+
+// Solves G^T W G x = b as gwg_cg32_mf describes.  Returns the iterations taken, or -1 when the mesh has no
+// cut into bricks that fit (more than about 600,000 elements on 152 SMs).
+int gwg_cg_whole(Context& c, const float* Wc, const float* dinv, const double* b, float* x, double rtol, int maxit) {
+    const MeshDesc& m = c.levels[0].mesh;
+    CgWhole a{};
+    size_t smem = 0;
+    if (!plan(c, a, &smem)) return -1;
     a.pitch = (m.nnx + 3) / 4 * 4;
     a.nny = m.nny;
     a.nn = a.pitch * m.nny * m.nnz;

@@ -49,6 +49,7 @@ int gwg_cg_mg(Context& c, const double* A, const double* dinv, const double* b, 
               double* work, double* scal);
 int gwg_cg_mg32(Context& c, const float* A, const float* dinv, const double* b, float* x, double rtol, int maxit,
                 float* work, double* scal);
+bool gwg_cg_whole_fits(Context& c);
 int gwg_cg32_mf(Context& c, const float* Wc, const float* dinv, const double* b, float* x, double rtol, int maxit,
                 float* work, double* scal);
 void gwg_mf_weights(Context& c, const double* W, float* Wc);
@@ -1037,17 +1038,17 @@ void Bsscr::run() {
             to_float(c, bw.p, bw32.p, nv);
             bwc32.ensure((size_t)mf_weights_size(c.mesh));
             gwg_mf_weights(c, bw.p, bwc32.p);   // the matrix-free inner operator's folded weights
-            // Jacobi inner solves: in 3D with an x extent the TMA kernel takes, the matrix-free apply at every
-            // size (us per launch against the FP32 stencil: 24^3 3.2 / 5.0, 64^3 4.9 / 8.2, 96^3 8.3 / 23.6,
-            // 128^3 16.7 / 54.8).  Else the FP32 stencil while it and the CG vectors take at most half
+            // Jacobi inner solves: in 3D the matrix-free apply on every mesh that the one-launch solve takes (solves with
+            // the stencil and with it: 18 x 14 x 22 37.5 / 33.5 ms, 30 x 30 x 34 129 / 116) and with an x extent the TMA kernel takes (us per launch against the FP32
+            // stencil: 24^3 3.2 / 5.0, 64^3 4.9 / 8.2, 96^3 8.3 / 23.6, 128^3 16.7 / 54.8).  Else the FP32 stencil while it and the CG vectors take at most half
             // of L2, then the plain matrix-free apply, which moves about a fifth of the bytes.
             // bfbt_inner_pc 2 / 3 force one form; the multigrid levels start from the FP32 stencil.
             int l2 = 0;
             UWG_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c.device));
             const double st_bytes = (double)npres * 4.0 * ((dim == 3 ? 27 : 9) + 6);
-            const bool tma_form = dim == 3 && c.mesh.nel[0] % 4 == 0;
+            const bool mf_form = dim == 3 && (c.mesh.nel[0] % 4 == 0 || (o.bfbt_inner_pc == 0 && gwg_cg_whole_fits(c)));
             stencil32 = o.bfbt_inner_pc == 2 ||
-                        ((o.bfbt_inner_pc == 0 || o.bfbt_inner_pc == 4) && !tma_form && st_bytes <= 0.5 * l2);
+                        ((o.bfbt_inner_pc == 0 || o.bfbt_inner_pc == 4) && !mf_form && st_bytes <= 0.5 * l2);
             const bool want_stencil32 = stencil32 || o.bfbt_inner_pc == 1;
             if (want_stencil32) bA32.ensure((size_t)(dim == 3 ? 27 : 9) * npres);
             gwg_stencil_fp32(c, bA.p, bd.p, want_stencil32 ? bA32.p : nullptr, bd32.p);

@@ -10,6 +10,8 @@
 // with coalesced stencil reads; the 57 MB FP64 stencil of a 64^3 mesh can stay in L2.  In FP32
 // the matrix-free chain is cheap, so the mixed form applies G^T W G matrix-free (k_cg_mf3_dir_tma,
 // k_cg_mf3_dir, k_cg_mf2_dir below) where that is faster than its FP32 stencil.
+// Up to about 600,000 elements a 3D matrix-free solve runs as one launch (cg_whole.cu) instead of the
+// two kernels per iteration described below.
 // Further down: the aggregation multigrid option for the inner solves, and the test and timing
 // hooks on the inner operator.
 //

@@ -1038,10 +1038,11 @@ void Bsscr::run() {
             to_float(c, bw.p, bw32.p, nv);
             bwc32.ensure((size_t)mf_weights_size(c.mesh));
             gwg_mf_weights(c, bw.p, bwc32.p);   // the matrix-free inner operator's folded weights
-            // Jacobi inner solves: in 3D the matrix-free apply on every mesh that the one-launch solve takes (solves with
-            // the stencil and with it: 18 x 14 x 22 37.5 / 33.5 ms, 30 x 30 x 34 129 / 116) and with an x extent the TMA kernel takes (us per launch against the FP32
-            // stencil: 24^3 3.2 / 5.0, 64^3 4.9 / 8.2, 96^3 8.3 / 23.6, 128^3 16.7 / 54.8).  Else the FP32 stencil while it and the CG vectors take at most half
-            // of L2, then the plain matrix-free apply, which moves about a fifth of the bytes.
+            // Jacobi inner solves: in 3D the matrix-free apply on every mesh that the one-launch solve takes (solves
+            // with the stencil and with it: 18 x 14 x 22 37.5 / 33.5 ms, 30 x 30 x 34 129 / 116) and with an x
+            // extent the TMA kernel takes (us per launch against the FP32 stencil: 24^3 3.2 / 5.0, 64^3 4.9 / 8.2,
+            // 96^3 8.3 / 23.6, 128^3 16.7 / 54.8).  Else the FP32 stencil while it and the CG vectors take at most
+            // half of L2, then the plain matrix-free apply, which moves about a fifth of the bytes.
             // bfbt_inner_pc 2 / 3 force one form; the multigrid levels start from the FP32 stencil.
             int l2 = 0;
             UWG_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c.device));

@@ -235,8 +235,8 @@ FAMILY_NOTES = {
     "apply": "one operator apply (k_apply): 27 stencil blocks of 3x3 per node, x read and y written once",
     "schur_pc": "one replay of the BFBt inner-CG graph = 12 iterations of k_cg_update + the direction kernel "
                 "(k_cg_spmv_dir on the 27-point G^T W G stencil, or the matrix-free FP32 kernel k_cg_mf3_dir_tma, "
-                "its element and weight planes staged by TMA, on meshes whose FP32 stencil would not fit in half "
-                "of L2); the roofline line is the direction kernel",
+                "its element and weight planes staged by TMA, on meshes "
+                "beyond the one-launch solve); the roofline line is the direction kernel",
     "learned": "U-Net corrections: tcgen05 implicit-GEMM convolutions (BF16, FP32 accumulate) and the head",
     "assembly": "rheology + moments per point, contraction of the moments into K_e (tensor core in the mixed forms)",
     "setup": "every launch of the solver's setup: node stencils from K_e, the Galerkin hierarchy and coarsest "

@@ -177,8 +177,10 @@ class _HostBuffers:
 
     A fresh array's pages are faulted in while the device copy writes them, at about 20 GB/s against 190 GB/s
     into pages that are present, so a call that returns 150 MB took longer to fault than to compute.  At most
-    LIMIT bytes are held; release() gives them back.  Safe from any thread and from garbage collection inside
-    a call (the lock is re-entrant and no list is iterated while it changes)."""
+    LIMIT bytes are held; release() gives them back.  Safe from any thread.  A garbage collection may start
+    inside any of these methods and run finalisers that give memory back or ask for some: no method waits for
+    the lock, so whoever holds it finds the list as it left it.  A call that does not get the lock takes fresh
+    memory, or leaves its block to the allocator."""
 
     LIMIT = 1 << 30
     SMALLEST = 1 << 20
@@ -198,7 +200,8 @@ class _HostBuffers:
                 pass
 
     def __init__(self):
-        self._lock = threading.RLock()
+        self._lock = threading.Lock()
+        self._dropping = False   # release() was asked for
         self._free = []
         self._held = 0
 
@@ -209,26 +212,43 @@ class _HostBuffers:
         if need < self.SMALLEST:
             return np.empty(shape, dtype)
         raw = None
-        with self._lock:
-            fits = [k for k in range(len(self._free)) if need <= self._free[k].nbytes <= 2 * need]
-            if fits:
-                raw = self._free.pop(min(fits, key=lambda k: self._free[k].nbytes))
-                self._held -= raw.nbytes
+        if self._lock.acquire(blocking=False):
+            try:
+                if not self._dropping:
+                    fits = [k for k in range(len(self._free)) if need <= self._free[k].nbytes <= 2 * need]
+                    if fits:
+                        raw = self._free.pop(min(fits, key=lambda k: self._free[k].nbytes))
+                        self._held -= raw.nbytes
+            finally:
+                self._unlock()
         if raw is None:
             raw = np.empty(need, np.uint8)
         return np.asarray(self._Block(self, raw, shape, dtype))
 
     def _give_back(self, raw):
-        with self._lock:
+        if not self._lock.acquire(blocking=False):
+            return
+        try:
             while self._free and self._held + raw.nbytes > self.LIMIT:
                 self._held -= self._free.pop(0).nbytes
             if self._held + raw.nbytes <= self.LIMIT:
                 self._free.append(raw)
                 self._held += raw.nbytes
+        finally:
+            self._unlock()
+
+    def _unlock(self):
+        if self._dropping:
+            self._free, self._held, self._dropping = [], 0, False
+        self._lock.release()
+        if self._dropping:   # asked for since the line above looked
+            self.release()
 
     def release(self):
-        with self._lock:
-            self._free, self._held = [], 0
+        """gives the held memory back; where another call is in progress, when that one ends"""
+        self._dropping = True
+        if self._lock.acquire(blocking=False):
+            self._unlock()
 
 
 host_buffers = _HostBuffers()

@@ -518,6 +518,15 @@ int uwgpu_bfbt_operator_apply(uwgpu_ctx* ctx, int32_t form, const double* x, dou
     });
 }
 
+int uwgpu_bfbt_inner_solve(uwgpu_ctx* ctx, int32_t form, double rtol, int32_t max_it, const double* b, double* x,
+                           int32_t* iterations) {
+    return guarded(ctx, [&](Context& c) {
+        UWG_REQUIRE(b && x, UWGPU_ERR_ARGUMENT, "b and x are required");
+        const int its = uwg::bfbt_inner_hook(c, form, rtol, max_it, b, x);
+        if (iterations) *iterations = its;
+    });
+}
+
 int uwgpu_jacobian_set(uwgpu_ctx* ctx, int32_t on) {
     return guarded(ctx, [&](Context& c) {
         UWG_REQUIRE(!on || (c.has_mesh && c.mesh.dim == 2), UWGPU_ERR_UNSUPPORTED,

@@ -16,14 +16,16 @@
 // The sums are exchanged by a warp of their own.  beta does not enter A z, so the other warps read the halo and
 // form A z while that warp waits for r.z; they wait for p.q.  An iteration is then bound by that one wait (a
 // store, its way through L2, the load that sees it and the sums: 1 to 2 us, growing with the blocks that poll),
-// the halo's, and the shared-memory reads of the stencil.  Measured per iteration, two launches -> one warp of
-// sixteen exchanging while the others wait -> this form: 64 x 80 x 112 elements 12.3 -> 7.5 -> 7.1 us, 64^3
-// 8.3 -> 6.0 -> 5.1, 32^3 -> 4.9 -> 3.6, 16^3 -> 3.7 -> 3.2.  Sixteen copies of the block sums, so that the blocks
-// do not all poll the same lines: 8.2 -> 7.5 us on the first mesh.
+// the halo's, and the shared-memory reads of the stencil.  Measured per iteration, with the sums in pairs of FP32
+// (below), two launches -> one warp of sixteen exchanging while the others wait -> this form: 64 x 80 x 112
+// elements 12.3 -> 7.5 -> 7.1 us, 64^3 8.3 -> 6.0 -> 5.1, 32^3 -> 4.9 -> 3.6, 16^3 -> 3.7 -> 3.2.  Sixteen copies
+// of the block sums, so that the blocks do not all poll the same lines: 8.2 -> 7.5 us on the first mesh.
 //
-// A thread's and a warp's sums are FP32, as in the two-kernel form; above that, where that form adds in
-// FP64, sums are unevaluated pairs of FP32 values (TwoSum, Knuth, The Art of Computer Programming vol. 2,
-// 4.2.2), about 48 bits, of which alpha and beta keep 24: an FP64 addition holds a warp for 64 cycles.
+// A thread's and a warp's sums are FP32 and all sums above a warp FP64, as in the two-kernel form: a sum over the
+// mesh may pass the largest FP32.  The thirteen dependent FP64 additions of a sum hold its warp for 64 cycles each;
+// as pairs of FP32 (48 bits, FP32 range) the same sums took 0.7 to 1.0 us less per iteration.  That is the price of
+// the precision: per iteration now 64 x 80 x 112 elements 7.9 us, 64^3 5.8, 32^3 4.6, 16^3 4.0.  (Additions with
+// half the lanes off at each level, and a division by an FP32 reciprocal and two corrections, gain nothing.)
 //
 // Every wait is bounded; a block whose wait ends without its word reports an error and returns.
 #include <algorithm>
@@ -45,7 +47,7 @@ constexpr int kWRim = 3;                 // nodes of the brick's upper faces per
 constexpr int kWHalo = 4;                // halo elements per thread at most
 constexpr int kWBlocks = 160;            // blocks at most: five sums per lane
 constexpr int kWCopies = 16;             // copies of the block sums, each read by a sixteenth of the blocks
-static_assert(2 * kWCopies <= 32 && kWWarps == 16, "one lane per word published, each holding the block's sum");
+static_assert(kWCopies <= 32 && kWWarps == 16, "one lane per word published, each holding the block's sum");
 constexpr int kWCheck = 12;              // iterations between convergence tests, as in the two-kernel form
 constexpr int kWPoll = 1 << 20;
 
@@ -64,7 +66,7 @@ struct CgWhole {
     const double* b;
     float* x;
     u64* face;                           // [element] {z, tag}
-    u64* sums;                           // [rz, pq, rr][copy][block][high, low part]
+    u64* sums;                           // [rz, pq, rr][copy][block] {sum, tag}
     double* report;                      // iterations, code, ||r||, ||b||
     int* failed;
     int maxit;
@@ -80,70 +82,58 @@ __device__ __forceinline__ u64 ld_word(const u64* p) {
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
     return w;
 }
-__device__ __forceinline__ void ld_words(const u64* p, u64& w0, u64& w1) {
-    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(p) : "memory");
+// a block sum and its tag in one aligned 16-byte word, read and written whole
+__device__ __forceinline__ void st_sum(u64* p, double v, uint32_t tag) {
+    asm volatile("{ .reg .b128 q; mov.b128 q, {%1, %2}; st.relaxed.gpu.global.b128 [%0], q; }" ::"l"(p),
+                 "l"(__double_as_longlong(v)), "l"((u64)tag)
+                 : "memory");
+}
+__device__ __forceinline__ void ld_sum(const u64* p, double& v, uint32_t& tag) {
+    u64 a, b;
+    asm volatile("{ .reg .b128 q; ld.relaxed.gpu.global.b128 q, [%2]; mov.b128 {%0, %1}, q; }" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+    v = __longlong_as_double((long long)a);
+    tag = (uint32_t)b;
 }
 __device__ __forceinline__ float word_value(u64 w) { return __uint_as_float((uint32_t)w); }
 
-// h + l += bh + bl.  Symmetric in its arguments, so all lanes of an xor tree get the same bits.
-__device__ __forceinline__ void add_pair(float& h, float& l, float bh, float bl) {
-    const float s = __fadd_rn(h, bh);
-    const float t = __fsub_rn(s, h);
-    const float e = __fadd_rn(__fsub_rn(h, __fsub_rn(s, t)), __fsub_rn(bh, t));
-    h = s;
-    l = __fadd_rn(__fadd_rn(l, bl), e);
-}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-// exchange warp: publishes the sum of the block's warp sums sw and adds those of all blocks; false when a
-// word does not come
-__device__ __forceinline__ bool global_sum(const float* sw, u64* slots, int blocks, uint32_t tag, float& h, float& l) {
+// exchange warp: publishes the sum of the block's warp sums sw and adds those of all blocks, every lane of every
+// block in the same order; false when a word does not come
+__device__ __forceinline__ bool global_sum(const float* sw, u64* slots, int blocks, uint32_t tag, double& sum) {
     const int lane = threadIdx.x & 31;
-    h = sw[lane % kWWarps];   // the two halves of the warp form the same sum
-    l = 0.f;
+    double v = (double)sw[lane % kWWarps];   // the two halves of the warp form the same sum
 #pragma unroll
-    for (int o = kWWarps / 2; o > 0; o >>= 1) {
-        const float bh = __shfl_xor_sync(0xffffffffu, h, o), bl = __shfl_xor_sync(0xffffffffu, l, o);
-        add_pair(h, l, bh, bl);
-    }
-    if (lane < 2 * kWCopies)
-        st_word(slots + 2 * (kWBlocks * (lane >> 1) + blockIdx.x) + (lane & 1), (lane & 1) == 0 ? h : l, tag);
+    for (int o = kWWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane < kWCopies) st_sum(slots + 2 * (kWBlocks * lane + blockIdx.x), v, tag);
     const u64* from = slots + 2 * kWBlocks * (blockIdx.x % kWCopies);
     constexpr int M = kWBlocks / 32;
-    u64 wh[M], wl[M];
+    double w[M];
+    uint32_t t[M];
     bool all = false;
     for (int tries = 0; tries < kWPoll && !all; ++tries) {
         bool mine = true;
 #pragma unroll
         for (int m = 0; m < M; ++m) {
             const int i = lane + 32 * m;
-            if (i < blocks) ld_words(from + 2 * i, wh[m], wl[m]);
-            else wh[m] = wl[m] = (u64)tag << 32;
+            w[m] = 0.0;
+            t[m] = tag;
+            if (i < blocks) ld_sum(from + 2 * i, w[m], t[m]);
         }
 #pragma unroll
-        for (int m = 0; m < M; ++m) mine = mine && (uint32_t)(wh[m] >> 32) == tag && (uint32_t)(wl[m] >> 32) == tag;
+        for (int m = 0; m < M; ++m) mine = mine && t[m] == tag;
         all = __all_sync(0xffffffffu, mine);
     }
-    h = 0.f;
-    l = 0.f;
+    v = w[0];
 #pragma unroll
-    for (int m = 0; m < M; ++m) add_pair(h, l, word_value(wh[m]), word_value(wl[m]));
+    for (int m = 1; m < M; ++m) v += w[m];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float bh = __shfl_xor_sync(0xffffffffu, h, o), bl = __shfl_xor_sync(0xffffffffu, l, o);
-        add_pair(h, l, bh, bl);
-    }
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    sum = v;
     return all;
-}
-// (ah + al) / (bh + bl) as FP32: the quotient of the leading parts and one correction by its remainder
-__device__ __forceinline__ float pair_ratio(float ah, float al, float bh, float bl) {
-    const float q = __fdiv_rn(ah, bh);
-    const float rem = fmaf(-q, bl, al) + fmaf(-q, bh, ah);
-    const float c = __fdiv_rn(rem, bh);
-    return isfinite(c) ? q + c : q;
 }
 
 // barrier of the whole block, and of the warps that hold elements
@@ -189,21 +179,20 @@ __global__ void __launch_bounds__(kWAll, 1) k_cg_whole(CgWhole a) {
     const int blocks = gridDim.x;
     // k = -1: z = 1/diag b, p = z, q = A z; then iteration k: x, r, z with alpha, r.z, p and q with beta, p.q
     if (warp == kWWarps) {
-        float rz_h = 0.f, rz_l = 0.f, pq_h, pq_l;   // r.z and p.q of the last sums
-        double norm0 = 0.0;
+        double rz = 0.0, norm0 = 0.0;
         sync_all();
         for (int k = -1;; ++k) {
             const uint32_t tag = (uint32_t)(k + 2);
             const bool check = k < 0 || (k + 1) % kWCheck == 0;
             sync_all();
-            float h, l, h2 = 0.f, l2 = 0.f;
-            bool ok = global_sum(sw, rz_slots, blocks, tag, h, l);
-            if (check) ok = global_sum(sw2, rr_slots, blocks, tag, h2, l2) && ok;
+            double rz_new, pq, rr = 0.0;
+            bool ok = global_sum(sw, rz_slots, blocks, tag, rz_new);
+            if (check) ok = global_sum(sw2, rr_slots, blocks, tag, rr) && ok;
             if (lane == 0) {
-                s_beta = k < 0 ? 0.f : pair_ratio(h, l, rz_h, rz_l);
+                s_beta = k < 0 ? 0.f : (float)(rz_new / rz);
                 if (!ok) s_fail = 1;
                 if (check) {
-                    const double norm = sqrt((double)h2 + (double)l2);
+                    const double norm = sqrt(rr);
                     if (k < 0) norm0 = norm;
                     const int code = !(norm0 > 0.0) ? 1 : !isfinite(norm) ? 2 : k >= 0 && norm <= a.rtol * norm0 ? 3
                                    : k + 1 >= a.maxit ? 4 : 0;
@@ -216,14 +205,13 @@ __global__ void __launch_bounds__(kWAll, 1) k_cg_whole(CgWhole a) {
                     }
                 }
             }
-            rz_h = h;
-            rz_l = l;
+            rz = rz_new;
             sync_all();
             if (s_fail || s_stop) break;
             sync_all();
-            ok = global_sum(sw, pq_slots, blocks, tag, pq_h, pq_l);
+            ok = global_sum(sw, pq_slots, blocks, tag, pq);
             if (lane == 0) {
-                s_alpha = pair_ratio(rz_h, rz_l, pq_h, pq_l);
+                s_alpha = (float)(rz / pq);
                 if (!ok) s_fail = 1;
             }
             sync_all();

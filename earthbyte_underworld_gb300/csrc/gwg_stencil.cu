@@ -1824,6 +1824,52 @@ void bfbt_operator_hook(Context& c, int form, const double* xh, double* yh, int 
     UWG_CUDA(cudaStreamSynchronize(c.stream));
 }
 
+// Test hook: x = A^{-1} b by the Jacobi-preconditioned inner CG in one of its forms: 0 the FP64 stencil, 1 the mixed
+// form's matrix-free solve (one launch where the mesh has a cut), 2 the FP32 stencil, 3 the matrix-free solve in
+// two kernels per iteration.  b has no constant part where A annihilates it.  Returns the iterations.
+int bfbt_inner_hook(Context& c, int form, double rtol, int maxit, const double* bh, double* xh) {
+    UWG_REQUIRE(c.operator_built, UWGPU_ERR_STATE, "the fine velocity operator is not built (solve first)");
+    UWG_REQUIRE(form >= 0 && form <= 3, UWGPU_ERR_ARGUMENT, "form must be 0 to 3");
+    UWG_REQUIRE(rtol > 0.0 && maxit > 0, UWGPU_ERR_ARGUMENT, "rtol and max_it must be positive");
+    const MeshDesc& m = c.levels[0].mesh;
+    const int64_t ne = m.ne, nb = m.dim == 3 ? 27 : 9;
+    UWG_REQUIRE(ne * nb < (int64_t)1 << 31, UWGPU_ERR_TOO_LARGE, "BFBt stencil: element count too large");
+    struct PlainJacobi {   // without the plane correction of an earlier solve
+        Context& c;
+        const bool was;
+        explicit PlainJacobi(Context& ctx) : c(ctx), was(ctx.cc.on) { c.cc.on = false; }
+        ~PlainJacobi() { c.cc.on = was; }
+    } plain(c);
+    DArray<double> W, A, dinv, b, x, work, scal;
+    DArray<float> W32, A32, dinv32, x32, work32;
+    W.ensure((size_t)m.nn * m.dim);
+    A.ensure((size_t)(nb * ne));
+    for (auto* v : {&dinv, &b, &x}) v->ensure((size_t)ne);
+    scal.ensure(8);
+    bfbt_weights(c, W.p);
+    gwg_stencil_build(c, W.p, A.p, dinv.p);
+    UWG_CUDA(cudaMemcpyAsync(b.p, bh, (size_t)ne * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    int its = 0;
+    if (form == 0) {
+        work.ensure((size_t)4 * ne);
+        its = gwg_cg(c, A.p, dinv.p, b.p, x.p, rtol, maxit, work.p, scal.p);
+    } else {
+        for (auto* v : {&dinv32, &x32}) v->ensure((size_t)ne);
+        work32.ensure((size_t)4 * ne);
+        A32.ensure((size_t)(nb * ne));
+        W32.ensure((size_t)mf_weights_size(m));
+        gwg_stencil_fp32(c, A.p, dinv.p, A32.p, dinv32.p);
+        gwg_mf_weights(c, W.p, W32.p);
+        if (form == 1) its = gwg_cg32_mf(c, W32.p, dinv32.p, b.p, x32.p, rtol, maxit, work32.p, scal.p);
+        else if (form == 2) its = gwg_cg32(c, A32.p, dinv32.p, b.p, x32.p, rtol, maxit, work32.p, scal.p);
+        else its = gwg_cg_T<float>(c, nullptr, W32.p, dinv32.p, b.p, x32.p, rtol, maxit, work32.p, scal.p);
+        to_double(c, x32.p, x.p, ne);
+    }
+    UWG_CUDA(cudaMemcpyAsync(xh, x.p, (size_t)ne * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    UWG_CUDA(cudaStreamSynchronize(c.stream));
+    return its;
+}
+
 // ---- multigrid hierarchy for G^T W G ----------------------------------------------------
 void dense_inverse(Context& c, double* M, int64_t n);                      // operator.cu
 template <typename T> void dense_apply(Context& c, const double* M, int64_t n, const T* b, T* x);

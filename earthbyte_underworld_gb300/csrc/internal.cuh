@@ -406,6 +406,7 @@ void weights_set(Context& c, int kind, const int32_t res[3]);
 void integration_points(Context& c, const double** xi, const double** w);
 void integration_points_download(Context& c, double* xi, double* w);
 void bfbt_operator_hook(Context& c, int form, const double* xh, double* yh, int iterations, double* ms);
+int bfbt_inner_hook(Context& c, int form, double rtol, int maxit, const double* bh, double* xh);
 int tc_check(int layout, int fmt, int N, int K, const uint16_t* A, const uint16_t* B, float* D);
 void advect_particles(Context& c, double dt, int order, bool fallback, uint32_t& fell_back, uint32_t& left_mesh);
 template <typename T> void level_cheb(Context&, Level&, const T*, T*, int, bool);

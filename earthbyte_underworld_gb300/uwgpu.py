@@ -143,6 +143,7 @@ def load(build_if_missing: bool = True):
         L.uwgpu_weights_set.argtypes = [P, C.c_int32, P]
         L.uwgpu_integration_points.argtypes = [P, P, P]
         L.uwgpu_time_bfbt_apply.argtypes = [P, C.c_int32, C.c_int32, P]
+        L.uwgpu_bfbt_inner_solve.argtypes = [P, C.c_int32, C.c_double, C.c_int32, P, P, P]
         L.uwgpu_launch_count.argtypes = [P]
         L.uwgpu_launch_count.restype = C.c_int64
         L.uwgpu_learned_create.argtypes = [P, C.c_int32, C.c_int32, C.c_uint64]
@@ -536,6 +537,15 @@ class Context:
         y = np.empty_like(x)
         self._check(self._L.uwgpu_bfbt_operator_apply(self._h, form, _ptr(x), _ptr(y)))
         return y
+
+    def bfbt_inner_solve(self, b, form=0, rtol=1e-4, max_it=500):
+        """(x, iterations) of the inner CG on that operator (form 0: FP64 stencil, 1: matrix-free FP32 as the mixed
+        form runs it, 2: FP32 stencil, 3: matrix-free FP32 in two kernels per iteration)"""
+        b = np.ascontiguousarray(b, dtype=np.float64)
+        x = np.empty_like(b)
+        its = C.c_int32()
+        self._check(self._L.uwgpu_bfbt_inner_solve(self._h, form, rtol, max_it, _ptr(b), _ptr(x), C.byref(its)))
+        return x, its.value
 
     def time_bfbt_apply(self, form=1, iterations=20):
         ms = C.c_double()

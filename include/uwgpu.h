@@ -408,6 +408,13 @@ int uwgpu_time_smooth(uwgpu_ctx* ctx, int32_t precision, int32_t sweeps, int32_t
  * inner CG's operator kernel in that form, elapsed device milliseconds in ms. */
 int uwgpu_bfbt_operator_apply(uwgpu_ctx* ctx, int32_t form, const double* x, double* y);
 int uwgpu_time_bfbt_apply(uwgpu_ctx* ctx, int32_t form, int32_t iterations, double* ms);
+/* Test hook on the inner solve of that preconditioner: x = A^{-1} b to ||b - A x|| <= rtol ||b|| by
+ * Jacobi-preconditioned CG, at most max_it iterations (in steps of twelve), `iterations` of them taken.
+ * form 0: the FP64 stencil; 1: the matrix-free FP32 solve as the mixed form runs it (one launch where
+ * the mesh allows it); 2: the FP32 stencil; 3: the matrix-free FP32 solve in two kernels per iteration.
+ * b and x are host arrays of one value per element; b has no constant part where A annihilates it. */
+int uwgpu_bfbt_inner_solve(uwgpu_ctx* ctx, int32_t form, double rtol, int32_t max_it, const double* b, double* x,
+                           int32_t* iterations);
 
 /* Tensor-core self-check (no reference counterpart): D = A B^T for A 128 x k and B n x k (row-major
  * 16-bit values: bfloat16 bits for format 1, IEEE half bits for format 0), D 128 x n FP32, computed

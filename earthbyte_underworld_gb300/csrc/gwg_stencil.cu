@@ -1653,17 +1653,12 @@ static int gwg_cg_T(Context& c, const T* A, const float* Wmf, const T* dinv, con
     // weights of about one node per element in place of the stencil)
     const double it_bytes = (double)ne * sizeof(T) * (8 + (Wmf ? m.dim : nb) + 5 + (cc ? 3 : 0));
     const double it_flops = Wmf ? (double)ne * (m.dim == 3 ? 110.0 : 46.0) : (double)ne * (2.0 * nb + 14.0);
-    // The next replay is queued before the last one's residual is known while that of the one before is
-    // more than kFar times the tolerance away (the residual falls by a few percent per replay), so the GPU
-    // does not wait for the host: a replay of 185 us used to be followed by 25 us of idle time.  Near the
-    // tolerance, and before anything is known, the host looks first; a replay queued in vain leaves x nearer
-    // to the solution.  The FP64 form stops exactly where the test says.
-    constexpr double kFar = sizeof(T) == 4 ? 4.0 : 1e300;
-    for (auto& ev : c.pcg_events)
-        if (!ev) UWG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    double* hs = c.host_scalars;
-    int it = 0, queued = 0, seen = 0;   // iterations and replays queued, replays whose residual has been read
-    auto queue = [&]() {
+    // The host looks at the residual after every replay: 25 us of idle time against a replay of 185 us on a mesh of
+    // 96^3.  With the next replay queued before that (2D 256^2 7.0 -> 6.8 us an iteration, 128^3 30.7 -> 30.4) the
+    // solve goes on past the solution; with x kept aside for that case the gain is gone.
+    double* h = c.host_scalars;
+    int it = 0;
+    while (it < maxit) {
         {
             LaunchScope ls(c, UWGPU_KERNEL_SCHUR_PC);
             UWG_CUDA(cudaGraphLaunch(pg->exec, c.stream));
@@ -1671,20 +1666,8 @@ static int gwg_cg_T(Context& c, const T* A, const float* Wmf, const T* dinv, con
         note_work(c, UWGPU_KERNEL_SCHUR_PC, block * it_bytes, block * it_flops);
         c.launches += (cc ? 5 : 2) * block - 1;
         it += block;
-        const int slot = queued++ & 1;
-        UWG_CUDA(cudaMemcpyAsync(hs + 8 * slot, scal, 8 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-        UWG_CUDA(cudaEventRecord(c.pcg_events[slot], c.stream));
-    };
-    double ratio = 0.0;   // last known ||r|| over its tolerance
-    while (true) {
-        if (queued == seen) {
-            if (it >= maxit) break;
-            queue();
-        }
-        if (it < maxit && ratio > kFar && queued == seen + 1) queue();
-        const double* h = hs + 8 * (seen & 1);
-        UWG_CUDA(cudaEventSynchronize(c.pcg_events[seen & 1]));
-        ++seen;
+        UWG_CUDA(cudaMemcpyAsync(h, scal, 8 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+        UWG_CUDA(cudaStreamSynchronize(c.stream));
         const double r0 = std::sqrt(h[7]);
         if (!(r0 > 0.0)) {   // nothing to solve: x = 0
             UWG_CUDA(cudaMemsetAsync(x, 0, (size_t)ne * sizeof(T), c.stream));
@@ -1693,7 +1676,6 @@ static int gwg_cg_T(Context& c, const T* A, const float* Wmf, const T* dinv, con
         const double rn = std::sqrt(h[6]);   // rr of the block's last iteration (k = 11: slot 5 + 1)
         if (!std::isfinite(rn)) throw Error(UWGPU_ERR_NAN, "NaN in the BFBt inner solve");
         if (rn <= rtol * r0) break;
-        ratio = rn / (rtol * r0);
     }
     check_launch("gwg_cg");
     return it;

@@ -294,7 +294,6 @@ struct Context {
     } cc;
     std::vector<PcgGraph> pcg_graphs;
     DArray<uint64_t> cg_words;   // words the blocks of the one-launch inner solve exchange
-    cudaEvent_t pcg_events[2] = {nullptr, nullptr};   // the residuals of two queued replays
 
     // learned velocity preconditioner (csrc/unet.cu), created on request
     unet::Net* net = nullptr;
@@ -303,8 +302,6 @@ struct Context {
         unet::destroy(net);
         for (auto& g : pcg_graphs)
             if (g.exec) cudaGraphExecDestroy(g.exec);
-        for (auto ev : pcg_events)
-            if (ev) cudaEventDestroy(ev);
     }
 };
 

@@ -45,3 +45,26 @@ def test_one_launch_sums_have_the_range_of_fp64(uw):
         big, its_big = ctx.bfbt_inner_solve(b * scale, form=1, rtol=1e-5)
     assert 24 <= its == its_big and np.isfinite(x).all() and np.abs(x).max() > 0
     assert np.array_equal(big, x * scale)
+
+
+@pytest.mark.parametrize("nel,form", [((16, 12), 2), ((10, 9, 8), 2), ((16, 12), 3), ((12, 9, 8), 3), ((10, 9, 8), 3),
+                                      ((68, 19, 21), 3), ((30, 31, 21), 3), ((12, 9, 8), 1), ((10, 9, 8), 0)])
+def test_inner_solve_stops_where_its_test_is_met(uw, nel, form):
+    """x meets the tolerance, and twelve iterations before the end it did not: each form, the two-kernel matrix-free
+    one with both of its direction kernels (x extents that are a multiple of 4 and not).  Tolerances that FP32
+    meets (the recurrence's residual is then that of x to a few 2^-24, so cases within 5% are left out)."""
+    seen = 0
+    with _uniform(uw, nel) as ctx:
+        b = np.random.default_rng(5).standard_normal(int(np.prod(nel)))
+        b = ctx.bfbt_operator_apply(b - b.mean())
+        for rtol in 10.0 ** -np.arange(1.0, 4.5, 0.125):
+            x, its = ctx.bfbt_inner_solve(b, form=form, rtol=rtol, max_it=480)
+            if its < 24:
+                continue
+            y, before = ctx.bfbt_inner_solve(b, form=form, rtol=rtol, max_it=its - 12)
+            res = [np.linalg.norm(b - ctx.bfbt_operator_apply(v)) / np.linalg.norm(b) / rtol for v in (x, y)]
+            assert before == its - 12 and res[0] < 1.05
+            if abs(res[1] - 1.0) > 0.05:
+                seen += 1
+                assert res[1] > 1.0, (rtol, its, res)
+    assert seen > 0

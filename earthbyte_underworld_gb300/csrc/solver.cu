@@ -1038,18 +1038,22 @@ void Bsscr::run() {
             to_float(c, bw.p, bw32.p, nv);
             bwc32.ensure((size_t)mf_weights_size(c.mesh));
             gwg_mf_weights(c, bw.p, bwc32.p);   // the matrix-free inner operator's folded weights
-            // Jacobi inner solves: in 3D the matrix-free apply on every mesh that the one-launch solve takes (solves
-            // with the stencil and with it: 18 x 14 x 22 37.5 / 33.5 ms, 30 x 30 x 34 129 / 116) and with an x
-            // extent the TMA kernel takes (us per launch against the FP32 stencil: 24^3 3.2 / 5.0, 64^3 4.9 / 8.2,
-            // 96^3 8.3 / 23.6, 128^3 16.7 / 54.8).  Else the FP32 stencil while it and the CG vectors take at most
-            // half of L2, then the plain matrix-free apply, which moves about a fifth of the bytes.
-            // bfbt_inner_pc 2 / 3 force one form; the multigrid levels start from the FP32 stencil.
+            // Jacobi inner solves: in 3D the matrix-free apply on every mesh that the one-launch solve takes.  Us per
+            // iteration in one launch / on the FP32 stencil / matrix-free in two kernels: 16^3 4.0 / 6.0 / 6.3,
+            // 18 x 14 x 22 4.0 / 6.0 / 6.1, 30 x 30 x 34 4.5 / 6.4 / 6.6, 64^3 5.9 / 11.4 / 10.5, 4 x 200 x 200
+            // 6.0 / 9.3 / 19.3.  Its products are also the nearer ones to FP64, as differences of z come before any
+            // rounded coefficient: error of A z against the FP64 stencil, matrix-free / FP32 stencil, on random z
+            // 6e-8 to 9e-8 / 1e-7, on the z of CG iterations 6e-8 / 8e-8, on smooth z 1e-7 to 3e-6 / 4e-7 to 5e-6
+            // (16^3 to 72^3, two-norm; 98 of 99 such pairs are smaller, one is 1.2 times larger).
+            // Else the FP32 stencil while it and the CG vectors take at most half of L2 (streamed from L2 it is the
+            // faster form), then the two-kernel matrix-free apply, which moves about a fifth of the bytes.
+            // bfbt_inner_pc 2 / 3 force one form; 4 has no one-launch solve; the multigrid levels of 1 start from
+            // the FP32 stencil.
             int l2 = 0;
             UWG_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c.device));
             const double st_bytes = (double)npres * 4.0 * ((dim == 3 ? 27 : 9) + 6);
-            const bool mf_form = dim == 3 && (c.mesh.nel[0] % 4 == 0 || (o.bfbt_inner_pc == 0 && gwg_cg_whole_fits(c)));
             stencil32 = o.bfbt_inner_pc == 2 ||
-                        ((o.bfbt_inner_pc == 0 || o.bfbt_inner_pc == 4) && !mf_form && st_bytes <= 0.5 * l2);
+                        ((o.bfbt_inner_pc == 4 || (o.bfbt_inner_pc == 0 && !gwg_cg_whole_fits(c))) && st_bytes <= 0.5 * l2);
             const bool want_stencil32 = stencil32 || o.bfbt_inner_pc == 1;
             if (want_stencil32) bA32.ensure((size_t)(dim == 3 ? 27 : 9) * npres);
             gwg_stencil_fp32(c, bA.p, bd.p, want_stencil32 ? bA32.p : nullptr, bd32.p);

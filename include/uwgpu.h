@@ -136,13 +136,15 @@ typedef struct {
     int32_t mg_cycle;         /* coarse corrections per level visit: 1 V-cycle (default), 2 W-cycle
                                  (-pc_mg_cycle_type v|w of the velocity PCMG)                */
     int32_t bfbt_inner_pc;    /* preconditioner of the scaled BFBt inner G^T W G solves: 0 Jacobi (default,
-                                 as the reference's KSP; the mixed form reads the FP32 stencil
-                                 while it fits in half of L2, else applies G^T W G matrix-free),
+                                 as the reference's KSP; the mixed form solves matrix-free in one
+                                 launch in 3D up to about 600,000 elements, else it reads the FP32
+                                 stencil while that fits in half of L2, else applies G^T W G
+                                 matrix-free),
                                  1 aggregation multigrid V-cycle, 2 Jacobi on the FP32 stencil,
                                  3 Jacobi with the matrix-free FP32 apply (2, 3: mixed form),
                                  4 Jacobi plus an additive coarse correction on the element
                                  checkerboards of single planes, Q1-P0's near-null pressure
-                                 modes (3D; the operator form chosen as for 0; 2D: as 0).  No
+                                 modes (3D, on the FP32 stencil or matrix-free; 2D: as 0).  No
                                  reference counterpart: the reference's inner KSP is Jacobi. */
 } uwgpu_solve_opts;
 

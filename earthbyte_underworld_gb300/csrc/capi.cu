@@ -527,6 +527,10 @@ int uwgpu_bfbt_inner_solve(uwgpu_ctx* ctx, int32_t form, double rtol, int32_t ma
     });
 }
 
+int uwgpu_cycle_give_up(uwgpu_ctx* ctx) {
+    return guarded(ctx, [&](Context& c) { c.cycle_give_up = true; });
+}
+
 int uwgpu_jacobian_set(uwgpu_ctx* ctx, int32_t on) {
     return guarded(ctx, [&](Context& c) {
         UWG_REQUIRE(!on || (c.has_mesh && c.mesh.dim == 2), UWGPU_ERR_UNSUPPORTED,

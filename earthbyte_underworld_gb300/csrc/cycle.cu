@@ -614,15 +614,18 @@ template <> const float* Dinv_of<float>(const Level& L) { return L.Dinv32.p; }
 double* vec(DArray<double>& d, DArray<float>&, double) { return d.p; }
 float* vec(DArray<double>&, DArray<float>& f, float) { return f.p; }
 
+void prepare(Context& c) {
+    if (c.cycle_bar.p) return;
+    c.cycle_bar.ensure(4);
+    UWG_CUDA(cudaMemsetAsync(c.cycle_bar.p, 0, 4 * sizeof(uint32_t), c.stream));
+    c.cycle_part.ensure((size_t)3 * kCyPass * kCyKrylovBlocks);
+}
+
 template <int DIM, typename T, bool HALF>
 void launch(Context& c, CyArgs<T>& a) {
     int sms = 0;
     UWG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
-    if (!c.cycle_bar.p) {
-        c.cycle_bar.ensure(4);
-        UWG_CUDA(cudaMemsetAsync(c.cycle_bar.p, 0, 4 * sizeof(uint32_t), c.stream));
-        c.cycle_part.ensure((size_t)3 * kCyPass * kCyKrylovBlocks);
-    }
+    prepare(c);
     a.bar = c.cycle_bar.p;
     a.which = c.cycle_which;
     a.part = c.cycle_part.p;
@@ -750,6 +753,13 @@ void cycle_fgmres_iteration(Context& c, const CycleOpts& o, const T* V, int k, i
     a.k = k;
     a.out = host_out;
     run<T>(c, a);
+}
+
+void cycle_begin(Context& c) {
+    if (c.cycle_give_up) prepare(c);
+    if (c.cycle_bar.p)
+        UWG_CUDA(cudaMemsetAsync(c.cycle_bar.p + 2, c.cycle_give_up ? 1 : 0, sizeof(uint32_t), c.stream));
+    c.cycle_give_up = false;
 }
 
 void cycle_check(Context& c) {

@@ -27,7 +27,10 @@ void cycle_run(Context& c, const CycleOpts& o, int first, const T* b, T* x);
 template <typename T>
 void cycle_fgmres_iteration(Context& c, const CycleOpts& o, const T* V, int k, int64_t n, T* z, T* w, T* vnext,
                             double* host_out);
-// Throws if a launch since the last check gave up on a barrier (synchronises the stream).
+// A launch that gives up on a barrier leaves a flag.  cycle_begin clears it at the start of a solve (an earlier one may
+// have ended early); cycle_check throws if it is set (synchronises the stream).  A solve that fails checks as well:
+// the values such a launch leaves unfinished make it fail in some other way sooner or later.
+void cycle_begin(Context& c);
 void cycle_check(Context& c);
 
 }  // namespace uwg

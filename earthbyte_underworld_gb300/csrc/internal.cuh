@@ -250,6 +250,7 @@ struct Context {
     DArray<uint32_t> cycle_bar;
     DArray<double> cycle_part;
     int cycle_which = 0;
+    bool cycle_give_up = false;      // test hook: the next solve's launches count as given up
     DArray<uint64_t> cycle_tagged;   // 2D iterates with the tags of the steps that formed them
     uint64_t cycle_tag = 1;          // next unused tag
     uint64_t cycle_layout[3] = {0, 0, 0};

@@ -1131,8 +1131,14 @@ void solve_bsscr(Context& c, const uwgpu_solve_opts& o, uwgpu_report& rep) {
     UWG_REQUIRE(o.learned_pc == 0 || o.learned_pc == 1, UWGPU_ERR_ARGUMENT, "bad learned_pc");
     UWG_REQUIRE(o.mg_cycle == 1 || o.mg_cycle == 2, UWGPU_ERR_ARGUMENT, "mg_cycle must be 1 (V) or 2 (W)");
     UWG_REQUIRE(o.bfbt_inner_pc >= 0 && o.bfbt_inner_pc <= 4, UWGPU_ERR_ARGUMENT, "bfbt_inner_pc must be 0..4");
-    Bsscr s(c, o, rep);
-    s.run();
+    cycle_begin(c);
+    try {
+        Bsscr s(c, o, rep);
+        s.run();
+    } catch (const Error&) {
+        cycle_check(c);
+        throw;
+    }
 }
 
 // Largest eigenvalue of Dinv A on the fine level for the Chebyshev smoother (timing hooks).
@@ -1152,7 +1158,7 @@ void estimate_fine_lmax(Context& c, const uwgpu_solve_opts& o) {
 // iterate gives one pair: inputs the residual r = b - K u and the V-cycle's answer V(r), target
 // the error left after that cycle, u* - u - V(r).  Late iterates carry the slowly converging
 // modes that a velocity solve spends its iterations on.  Returns the number of pairs.
-int learned_generate(Context& c, const uwgpu_solve_opts& o, int nsamples, uint64_t seed) {
+static int generate_pairs(Context& c, const uwgpu_solve_opts& o, int nsamples, uint64_t seed) {
     UWG_REQUIRE(c.assembled, UWGPU_ERR_STATE, "training data requested before assembly");
     UWG_REQUIRE(c.net != nullptr, UWGPU_ERR_STATE, "no network (uwgpu_learned_create)");
     UWG_REQUIRE(c.net->nn == c.mesh.nn, UWGPU_ERR_STATE, "the network was built for another mesh");
@@ -1198,6 +1204,16 @@ int learned_generate(Context& c, const uwgpu_solve_opts& o, int nsamples, uint64
     cycle_check(c);
     unet::dataset_finish(c, n);
     return n.nsamples;
+}
+
+int learned_generate(Context& c, const uwgpu_solve_opts& o, int nsamples, uint64_t seed) {
+    cycle_begin(c);
+    try {
+        return generate_pairs(c, o, nsamples, seed);
+    } catch (const Error&) {
+        cycle_check(c);
+        throw;
+    }
 }
 
 }  // namespace uwg

@@ -144,6 +144,7 @@ def load(build_if_missing: bool = True):
         L.uwgpu_integration_points.argtypes = [P, P, P]
         L.uwgpu_time_bfbt_apply.argtypes = [P, C.c_int32, C.c_int32, P]
         L.uwgpu_bfbt_inner_solve.argtypes = [P, C.c_int32, C.c_double, C.c_int32, P, P, P]
+        L.uwgpu_cycle_give_up.argtypes = [P]
         L.uwgpu_launch_count.argtypes = [P]
         L.uwgpu_launch_count.restype = C.c_int64
         L.uwgpu_learned_create.argtypes = [P, C.c_int32, C.c_int32, C.c_uint64]
@@ -546,6 +547,10 @@ class Context:
         its = C.c_int32()
         self._check(self._L.uwgpu_bfbt_inner_solve(self._h, form, rtol, max_it, _ptr(b), _ptr(x), C.byref(its)))
         return x, its.value
+
+    def cycle_give_up(self):
+        """test hook: the next solve's one-launch cycles count as having given up on a barrier"""
+        self._check(self._L.uwgpu_cycle_give_up(self._h))
 
     def time_bfbt_apply(self, form=1, iterations=20):
         ms = C.c_double()

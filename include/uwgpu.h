@@ -418,6 +418,10 @@ int uwgpu_time_bfbt_apply(uwgpu_ctx* ctx, int32_t form, int32_t iterations, doub
 int uwgpu_bfbt_inner_solve(uwgpu_ctx* ctx, int32_t form, double rtol, int32_t max_it, const double* b, double* x,
                            int32_t* iterations);
 
+/* Test hook on the one-launch multigrid cycle, whose waits are bounded: the launches of the next solve count as if one
+ * had given up on a barrier. */
+int uwgpu_cycle_give_up(uwgpu_ctx* ctx);
+
 /* Tensor-core self-check (no reference counterpart): D = A B^T for A 128 x k and B n x k (row-major
  * 16-bit values: bfloat16 bits for format 1, IEEE half bits for format 0), D 128 x n FP32, computed
  * by one tcgen05 MMA sequence with the operands staged in shared memory in the layout `layout`

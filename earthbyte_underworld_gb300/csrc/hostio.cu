@@ -4,7 +4,7 @@
 // the host arrays of the C ABI are by node, slot and element.  The change of layout runs on the device, at
 // memory bandwidth, on its way to or from a plain copy: done on the host (a scalar loop over a temporary) it
 // took most of a call: 40 of 44 ms for the element matrices of a 32^3 mesh, 7 of 8.6 ms for the mapping of
-// 2.4M points.  Staging memory is bounded: larger transfers go in pieces of kIoBytes.
+// 2.4M points.  Staging memory is bounded: larger transfers, either way, go in pieces of kIoBytes.
 #include <algorithm>
 
 #include "internal.cuh"
@@ -15,12 +15,13 @@ namespace {
 
 constexpr size_t kIoBytes = (size_t)64 << 20;
 
+// the components of nodes first + i, i < count, of n
 template <int DIM, typename T>
-__global__ void k_from_nodes(int64_t n, const double* __restrict__ a, T* __restrict__ soa) {
+__global__ void k_from_nodes(int64_t n, int64_t first, int64_t count, const double* __restrict__ a, T* __restrict__ soa) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= count) return;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) soa[(int64_t)d * n + i] = (T)a[i * DIM + d];
+    for (int d = 0; d < DIM; ++d) soa[(int64_t)d * n + first + i] = (T)a[i * DIM + d];
 }
 
 // out[i][0 .. W) of items first + i, i < count: the DIM components, then zeros
@@ -90,12 +91,15 @@ void in_pieces(Context& c, int64_t items, int64_t width, double* host, F&& make)
 template <typename T>
 void vector_from_host(Context& c, int64_t n, int dim, const double* host, T* soa) {
     if (n == 0) return;
-    c.io.ensure((size_t)(n * dim));
-    UWG_CUDA(cudaMemcpyAsync(c.io.p, host, (size_t)(n * dim) * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-    {
+    const int64_t step = (int64_t)(kIoBytes / (sizeof(double) * (size_t)dim));
+    c.io.ensure((size_t)(std::min(n, step) * dim));
+    for (int64_t first = 0; first < n; first += step) {
+        const int64_t count = std::min(step, n - first);
+        UWG_CUDA(cudaMemcpyAsync(c.io.p, host + first * dim, (size_t)(count * dim) * sizeof(double), cudaMemcpyHostToDevice,
+                                 c.stream));
         LaunchScope ls(c, -1);
-        if (dim == 3) k_from_nodes<3, T><<<blocks_for(n, 256), 256, 0, c.stream>>>(n, c.io.p, soa);
-        else k_from_nodes<2, T><<<blocks_for(n, 256), 256, 0, c.stream>>>(n, c.io.p, soa);
+        if (dim == 3) k_from_nodes<3, T><<<blocks_for(count, 256), 256, 0, c.stream>>>(n, first, count, c.io.p, soa);
+        else k_from_nodes<2, T><<<blocks_for(count, 256), 256, 0, c.stream>>>(n, first, count, c.io.p, soa);
     }
     check_launch("k_from_nodes");
 }

@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import threading
+import types
 
 import numpy as np
 
@@ -145,6 +146,14 @@ def load(build_if_missing: bool = True):
         L.uwgpu_time_bfbt_apply.argtypes = [P, C.c_int32, C.c_int32, P]
         L.uwgpu_bfbt_inner_solve.argtypes = [P, C.c_int32, C.c_double, C.c_int32, P, P, P]
         L.uwgpu_cycle_give_up.argtypes = [P]
+        L.uwgpu_hostmem_create.argtypes = [C.c_size_t, C.c_size_t]
+        L.uwgpu_hostmem_create.restype = P
+        L.uwgpu_hostmem_limit.argtypes = [P, C.c_size_t]
+        L.uwgpu_hostmem_limit.restype = None
+        L.uwgpu_hostmem_release.argtypes = [P]
+        L.uwgpu_hostmem_release.restype = None
+        L.uwgpu_hostmem_held.argtypes = [P, P, C.c_size_t]
+        L.uwgpu_hostmem_held.restype = C.c_size_t
         L.uwgpu_launch_count.argtypes = [P]
         L.uwgpu_launch_count.restype = C.c_int64
         L.uwgpu_learned_create.argtypes = [P, C.c_int32, C.c_int32, C.c_uint64]
@@ -174,85 +183,100 @@ def _ptr(a):
     return None if a is None else a.ctypes.data
 
 
+class _NumpyAllocator(C.Structure):
+    """numpy's PyDataMem_Handler (its C-API since 1.22)"""
+    _fields_ = [("name", C.c_char * 127), ("version", C.c_uint8), ("ctx", C.c_void_p), ("malloc", C.c_void_p),
+                ("calloc", C.c_void_p), ("realloc", C.c_void_p), ("free", C.c_void_p)]
+
+
+def _numpy_set_handler():
+    """numpy's PyDataMem_SetHandler, or None where this numpy has none"""
+    try:
+        from numpy._core import _multiarray_umath as umath
+    except ImportError:
+        from numpy.core import _multiarray_umath as umath
+    pointer = C.pythonapi.PyCapsule_GetPointer
+    pointer.restype, pointer.argtypes = C.c_void_p, [C.py_object, C.c_char_p]
+    table = C.cast(pointer(umath._ARRAY_API, None), C.POINTER(C.c_void_p))
+    if C.PYFUNCTYPE(C.c_uint)(table[211])() < 15:   # PyArray_GetNDArrayCFeatureVersion: 15 is numpy 1.22
+        return None
+    return C.PYFUNCTYPE(C.py_object, C.py_object)(table[304])
+
+
 class _HostBuffers:
-    """Memory of large result arrays, reused once the caller has dropped them.
+    """Arrays for large results, in memory that is reused once the caller has dropped them (csrc/hostmem.cu says what
+    that gains).  The arrays are ordinary ones that own their data: numpy allocates them from a pool of the library
+    and gives their memory back to it.  At most LIMIT bytes are kept; release() gives them back.  Safe from any
+    thread, and from garbage collections and finalisers, as the pool runs no Python code."""
 
-    A fresh array's pages are faulted in while the device copy writes them, at about 20 GB/s against 190 GB/s
-    into pages that are present, so a call that returns 150 MB took longer to fault than to compute.  At most
-    LIMIT bytes are held; release() gives them back.  Safe from any thread.  A garbage collection may start
-    inside any of these methods and run finalisers that give memory back or ask for some: no method waits for
-    the lock, so whoever holds it finds the list as it left it.  A call that does not get the lock takes fresh
-    memory, or leaves its block to the allocator."""
-
-    LIMIT = 1 << 30
     SMALLEST = 1 << 20
-
-    class _Block:
-        """Owner of one result's memory; numpy keeps it alive as the array's base."""
-
-        def __init__(self, pool, raw, shape, dtype):
-            self.pool, self.raw = pool, raw
-            self.__array_interface__ = dict(version=3, shape=shape, typestr=np.dtype(dtype).str,
-                                            data=(raw.ctypes.data, False))
-
-        def __del__(self):
-            try:
-                self.pool._give_back(self.raw)
-            except Exception:   # interpreter shutdown: the memory goes with the process
-                pass
+    _HANDLER = b"mem_handler"
 
     def __init__(self):
-        self._lock = threading.Lock()
-        self._dropping = False   # release() was asked for
-        self._free = []
-        self._held = 0
+        self._pool = None
+        self._limit = 1 << 30
+
+    @property
+    def LIMIT(self):
+        return self._limit
+
+    @LIMIT.setter
+    def LIMIT(self, nbytes):
+        self._limit = nbytes
+        if self._pool:
+            self._L.uwgpu_hostmem_limit(self._pool, nbytes)
+
+    def _open(self):
+        self._L = L = load()
+        self._set = _numpy_set_handler()
+        pool = L.uwgpu_hostmem_create(self._limit, self.SMALLEST)
+        at = [C.cast(f, C.c_void_p).value for f in (L.uwgpu_hostmem_malloc, L.uwgpu_hostmem_calloc,
+                                                    L.uwgpu_hostmem_realloc, L.uwgpu_hostmem_free)]
+        # arrays may outlive this object: what numpy calls stays for the life of the process
+        handler = _NumpyAllocator(b"uwgpu", 1, pool, *at)
+        _handlers.append(handler)
+        new = C.pythonapi.PyCapsule_New
+        new.restype, new.argtypes = C.py_object, [C.c_void_p, C.c_char_p, C.c_void_p]
+        self._capsule = new(C.addressof(handler), self._HANDLER, None)
+        self._pool = pool   # (two threads that come here at once make two pools, of which one is used)
 
     def array(self, shape, dtype):
         """an uninitialised C-ordered array"""
         shape = (shape,) if np.isscalar(shape) else tuple(shape)
-        need = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
-        if need < self.SMALLEST:
+        if int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize < self.SMALLEST:
             return np.empty(shape, dtype)
-        raw = None
-        if self._lock.acquire(blocking=False):
-            try:
-                if not self._dropping:
-                    fits = [k for k in range(len(self._free)) if need <= self._free[k].nbytes <= 2 * need]
-                    if fits:
-                        raw = self._free.pop(min(fits, key=lambda k: self._free[k].nbytes))
-                        self._held -= raw.nbytes
-            finally:
-                self._unlock()
-        if raw is None:
-            raw = np.empty(need, np.uint8)
-        return np.asarray(self._Block(self, raw, shape, dtype))
-
-    def _give_back(self, raw):
-        if not self._lock.acquire(blocking=False):
-            return
+        if not self._pool:
+            self._open()
+        if self._set is None:
+            return np.empty(shape, dtype)
+        before = self._set(self._capsule)   # (of this thread's context)
         try:
-            while self._free and self._held + raw.nbytes > self.LIMIT:
-                self._held -= self._free.pop(0).nbytes
-            if self._held + raw.nbytes <= self.LIMIT:
-                self._free.append(raw)
-                self._held += raw.nbytes
+            return np.empty(shape, dtype)
         finally:
-            self._unlock()
+            self._set(before)
 
-    def _unlock(self):
-        if self._dropping:
-            self._free, self._held, self._dropping = [], 0, False
-        self._lock.release()
-        if self._dropping:   # asked for since the line above looked
-            self.release()
+    def _sizes(self):
+        if not self._pool:
+            return []
+        L = self._L
+        sizes = (C.c_size_t * L.uwgpu_hostmem_held(self._pool, None, 0))()
+        return list(sizes[:L.uwgpu_hostmem_held(self._pool, sizes, len(sizes))])
+
+    @property
+    def _held(self):
+        return sum(self._sizes())
+
+    @property
+    def _free(self):
+        return [types.SimpleNamespace(nbytes=n) for n in self._sizes()]
 
     def release(self):
-        """gives the held memory back; where another call is in progress, when that one ends"""
-        self._dropping = True
-        if self._lock.acquire(blocking=False):
-            self._unlock()
+        """gives the kept memory back"""
+        if self._pool:
+            self._L.uwgpu_hostmem_release(self._pool)
 
 
+_handlers = []
 host_buffers = _HostBuffers()
 
 

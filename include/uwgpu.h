@@ -18,6 +18,7 @@
 #ifndef UWGPU_H
 #define UWGPU_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -417,6 +418,21 @@ int uwgpu_time_bfbt_apply(uwgpu_ctx* ctx, int32_t form, int32_t iterations, doub
  * b and x are host arrays of one value per element; b has no constant part where A annihilates it. */
 int uwgpu_bfbt_inner_solve(uwgpu_ctx* ctx, int32_t form, double rtol, int32_t max_it, const double* b, double* x,
                            int32_t* iterations);
+
+/* Host memory for large results, reused: an allocator whose freed blocks of `smallest` bytes and more are kept, up to
+ * `limit` bytes in all, and handed out again where at least half of a block is used (present pages are written about
+ * ten times as fast as fresh ones).  The pool lives as long as the process.  The last four have the arguments of
+ * numpy's data allocator; any thread may call them at any time.  uwgpu_hostmem_held: the number of kept blocks, and
+ * the sizes of the first `count`; uwgpu_hostmem_release gives them all back. */
+typedef struct uwgpu_hostmem uwgpu_hostmem;
+uwgpu_hostmem* uwgpu_hostmem_create(size_t limit, size_t smallest);
+void uwgpu_hostmem_limit(uwgpu_hostmem* pool, size_t limit);
+void uwgpu_hostmem_release(uwgpu_hostmem* pool);
+size_t uwgpu_hostmem_held(uwgpu_hostmem* pool, size_t* sizes, size_t count);
+void* uwgpu_hostmem_malloc(uwgpu_hostmem* pool, size_t size);
+void* uwgpu_hostmem_calloc(uwgpu_hostmem* pool, size_t count, size_t size);
+void* uwgpu_hostmem_realloc(uwgpu_hostmem* pool, void* block, size_t size);
+void uwgpu_hostmem_free(uwgpu_hostmem* pool, void* block, size_t size);
 
 /* Test hook on the one-launch multigrid cycle, whose waits are bounded: the launches of the next solve count as if one
  * had given up on a barrier. */

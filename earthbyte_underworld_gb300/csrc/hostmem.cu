@@ -37,13 +37,14 @@ struct uwgpu_hostmem {
 
 namespace {
 
-// large fresh blocks on large pages, as numpy asks for its own
+// Large fresh blocks ask for large pages exactly as numpy's own arrays do: from the next multiple of 4 KB, which a
+// kernel with larger base pages refuses.
 void* fresh(size_t size) noexcept {
-    constexpr size_t kLarge = (size_t)4 << 20, kPage = (size_t)2 << 20;
+    constexpr size_t kLarge = (size_t)4 << 20, kPage = 4096;
     void* p = std::malloc(size ? size : 1);
     if (p && size >= kLarge) {
-        const uintptr_t from = ((uintptr_t)p + kPage - 1) / kPage * kPage, to = ((uintptr_t)p + size) / kPage * kPage;
-        if (to > from) (void)madvise((void*)from, to - from, MADV_HUGEPAGE);
+        const size_t skip = kPage - (uintptr_t)p % kPage;
+        (void)madvise(static_cast<char*>(p) + skip, size - skip, MADV_HUGEPAGE);
     }
     return p;
 }

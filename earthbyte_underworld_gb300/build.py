@@ -36,7 +36,7 @@ def _stale(obj, src):
     if not os.path.exists(obj):
         return True
     deps = [src, os.path.join(HERE, "..", "include", "uwgpu.h")]
-    deps += [os.path.join(CSRC, h) for h in ("internal.cuh", "tc.cuh", "stencil.cuh", "cycle.cuh", "locate.cuh", "longsum.cuh")]
+    deps += [os.path.join(CSRC, h) for h in ("internal.cuh", "tc.cuh", "stencil.cuh", "cycle.cuh", "locate.cuh", "longsum.cuh", "unet.cuh")]
     t = os.path.getmtime(obj)
     return any(os.path.getmtime(d) > t for d in deps)
 

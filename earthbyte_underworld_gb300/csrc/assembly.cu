@@ -480,7 +480,7 @@ struct Tables3 {
 
 // Coefficient of moment m = 9a + 3b + c in table q (the ordering of Tables3 flattened:
 // Dxx, Dyy, Dzz as [t1][t2], then Mxy, Mxz, Myz as [ta][tb][to]); the same combinations
-// tables_from_moments forms.  Values are 0, +-1, +-2, +-4.
+// form_tables forms.  Values are 0, +-1, +-2, +-4.
 __host__ __device__ inline int table_coefficient(int q, int m) {
     const int Q[3][3] = {{1, 2, 1}, {1, -2, 1}, {1, 0, -1}};
     const int L[2][2] = {{1, 1}, {1, -1}};

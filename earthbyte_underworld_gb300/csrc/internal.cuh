@@ -255,7 +255,7 @@ struct Context {
     uint64_t cycle_tag = 1;          // next unused tag
     uint64_t cycle_layout[3] = {0, 0, 0};
     DArray<double> io;        // staging of transfers to and from the host (hostio.cu)
-    DArray<double> io_x, io_y;   // vectors of uwgpu_operator_apply
+    DArray<double> io_x, io_y;   // vectors of uwgpu_operator_apply, kept for the next call
     double* host_scalars = nullptr;   // pinned
 
     bool profiling = false;
